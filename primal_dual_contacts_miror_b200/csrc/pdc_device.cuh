@@ -139,14 +139,30 @@ struct CtaTeam {
     int rank, size, slot;
     BlockReducer<16> red;
     int* s_int;  // shared: [0] carry, [1..32] warp partials
-    __device__ CtaTeam(double* red_smem, int* int_smem) {
+    uint32_t* s_adj;  // shared: node adjacency of the symbolic factorisation
+    unsigned int parity = 0;
+    __device__ CtaTeam(double* red_smem, int* int_smem, uint32_t* adj_smem) {
         rank = threadIdx.x;
         size = blockDim.x;
         slot = blockIdx.x;
         red.init(red_smem);
         s_int = int_smem;
+        s_adj = adj_smem;
     }
     __device__ __forceinline__ void sync() { __syncthreads(); }
+    __device__ __forceinline__ uint32_t* adjacency(uint32_t*) const { return s_adj; }
+    __device__ __forceinline__ bool any(bool p) { return __syncthreads_or(p) != 0; }
+    // minimum over the team, one barrier (two alternating rows of warp slots)
+    __device__ __forceinline__ unsigned min_u32(unsigned v) {
+        __shared__ unsigned s_min[2][32];
+        const int lane = rank & 31;
+        unsigned* row = s_min[parity];
+        parity ^= 1;
+        v = __reduce_min_sync(0xffffffffu, v);
+        if (lane == 0) row[rank >> 5] = v;
+        __syncthreads();
+        return __reduce_min_sync(0xffffffffu, lane < (size >> 5) ? row[lane] : 0xffffffffu);
+    }
     template <int N>
     __device__ __forceinline__ void sum(double (&v)[N]) { red.sum(v); }
     template <int N>
@@ -199,6 +215,12 @@ struct WarpTeam {
         slot = slot_;
     }
     __device__ __forceinline__ void sync() { __syncwarp(); }
+    __device__ __forceinline__ uint32_t* adjacency(uint32_t* scratch) const { return scratch; }
+    __device__ __forceinline__ bool any(bool p) { return __any_sync(0xffffffffu, p) != 0; }
+    __device__ __forceinline__ unsigned min_u32(unsigned v) {
+        __syncwarp();  // a barrier, as the thread block's
+        return __reduce_min_sync(0xffffffffu, v);
+    }
     template <int N>
     __device__ __forceinline__ void sum(double (&v)[N]) {
 #pragma unroll

@@ -169,21 +169,15 @@ constexpr int kSparseWords = kSparseMax / 32;
 // the direct branch never leaves the factor for lack of room (a settled heap of
 // 256 boxes fills in to several thousand blocks)
 constexpr int kRowCap = kSparseMax * (kSparseMax - 1) / 2;
-// bytes of a slot's fixed part (bitsets, index arrays, node blocks and vectors;
-// the layout of SceneSolver::sparse_ws), before its off-diagonal blocks
-constexpr long long kSparseHeaderBytes = 4LL * (kSparseMax * kSparseWords + 6LL * kSparseMax + 10LL * (kSparseMax + 8) +
-                                                kRowCap + 8) +
-                                         8LL * (2 * 36 + 4 * 6) * kSparseMax;
-// An elimination level of the block team's factor is "fat" when one of its
-// columns takes more than kFatWork 6x6 block products (the sum of the pattern
-// sizes of the columns in its row list): such levels spread every column's
-// block rows over the team instead of one thread per column.
-constexpr int kFatWork = 24;
-// Bottom subtrees of the block team's elimination tree whose columns take at
-// most kSubWork block products in all are factored and swept by one thread
-// each, in elimination order, with no barrier; the nodes above them are
-// scheduled level by level.
-constexpr int kSubWork = 64;
+// 6x6 blocks of a factor: the off-diagonal ones and a diagonal one per node
+constexpr int kBlockCap = kRowCap + kSparseMax;
+// doubles of a packed inverse diagonal factor, padded to a multiple of 16 bytes
+constexpr int kInvStride = 22;
+// bytes of a slot before its blocks (bitsets, index arrays, inverse diagonal
+// factors and node vectors; the layout of SceneSolver::direct_ws)
+constexpr long long kSparseHeaderBytes = 4LL * (3LL * kSparseMax * kSparseWords + 13LL * (kSparseMax + 8) +
+                                                kBlockCap + 8) +
+                                         2LL * kBlockCap + 8LL * (kInvStride + 2 * 6 + 36) * kSparseMax;
 
 // The large-scene teams (whole GPU, one cluster) solve one scene per launch and
 // factor up to kSparseMaxLarge active bodies: the whole direct branch, which
@@ -781,7 +775,11 @@ class SceneSolver {
             T.sync();
             // rhs = sum getTrans(j) K^-1 sf - ru; block-Jacobi blocks; PCG start
             double rr[3] = {0, 0, 0};  // r.z, b.b, |D b|^2 (iterative branch)
-            for (int i = tid; i < n_local; i += nt) {
+            const bool rows_mode = !kLargeTeam && dense_mode;
+            if constexpr (!kLargeTeam) {
+                if (dense_mode) assemble_rows(eps);
+            }
+            for (int i = rows_mode ? n_local : tid; i < n_local; i += nt) {
                 const int gb = B.lbody[b0 + i];
                 if (!active(gb)) continue;
                 double gth[6];
@@ -831,8 +829,8 @@ class SceneSolver {
                         B.dsc[6 * gb + r] = d;
                         rr[2] += (d * rb[r]) * (d * rb[r]);
                     }
-                if (dense_mode) {
-                    assemble_dense_rows(gb, P);
+                if (kLargeTeam && dense_mode) {
+                    if constexpr (kLargeTeam) assemble_dense_rows(gb, P);
                 } else {
                     double* Pi = B.pinv + 21 * gb;
                     if (!spd6_inverse(P, Pi)) {
@@ -844,7 +842,8 @@ class SceneSolver {
                 }
                 for (int r = 0; r < 6; ++r) rr[1] += rb[r] * rb[r];
             }
-            T.sum(rr);  // sync: rhs, pinv complete
+            if (rows_mode) T.sync();
+            else T.sum(rr);  // sync: rhs, pinv complete
             const double bnorm = sqrt(rr[1]);
             // AMGCL's relative residual is measured in the scaled system: |D r| / |D b|
             const double bn = direct ? bnorm : sqrt(rr[2]);
@@ -860,7 +859,8 @@ class SceneSolver {
             int iters = 0;
             bool lin_bad = false;
             if (dense_mode) {
-                lin_bad = !dense_solve();
+                if constexpr (kLargeTeam) lin_bad = !dense_solve_warp();
+                else lin_bad = !direct_solve();
             }
             // mixed precision: FP32 PCG with FP64 refinement where PCG runs; an
             // inner breakdown or a refinement that stops converging falls back
@@ -1084,134 +1084,129 @@ class SceneSolver {
     }
 
     // ------------------------------------------- sparse direct solve (direct branch)
-    // Per-team scratch: bitset adjacency / column patterns, elimination order,
-    // block-column offsets, diagonal blocks, their Cholesky factors, the L blocks
-    // and three node vectors.  Node i is the i-th active body of the scene.
+    // Scratch of the large-scene teams (one slot, B.sparse_big): bitset adjacency
+    // / column patterns, elimination order, block-column offsets, diagonal
+    // blocks, their Cholesky factors, the L blocks and node vectors.  Node i is
+    // the i-th active body of the scene.
     struct Sparse {
-        uint32_t* adj;   // [kSparseMax][kSparseWords]
+        uint32_t* adj;   // [kSpMax][kSpWords]
+        uint32_t* radj;  // [kSpMax][kSpWords] row patterns, bit k = column eliminated k-th
         int* perm;       // elimination position -> node
         int* ipos;       // node -> elimination position
-        int* cstart;     // [kSparseMax + 1] first L block of each node's column
+        int* cstart;     // [n + 1] first L block of each node's column
         int* lvl_nodes;  // nodes grouped by elimination-tree height
-        int* height;     // [kSparseMax] elimination-tree height of each node
+        int* height;     // elimination-tree height of each node
         int* lvl_start;  // [levels + 1]
-        int* rowptr;     // [kSparseMax + 1] row lists: columns d with L(v, d) != 0
-        int* rowbase;    // [kSparseMax + 1] block team: first block row of each lvl_nodes position
-        int* lvl_mode;   // [levels] block team: 1 = fat level
-        int* sub_start;  // [team size + 1] block team: each thread's range of sub_nodes
-        int* sub_nodes;  // bottom-subtree nodes, grouped by thread, in elimination order
-        int* etp;        // elimination-tree parent (-1: root)
-        int* swork;      // subtree work (block products)
-        int* thr;        // thread of a bottom-subtree node, -1 above them
-        int* rowidx;     // [kRowCap]
-        int* meta;       // [0] number of levels
-        double* Dg;      // [kSparseMax][36] diagonal blocks
-        double* Ld;      // [kSparseMax][36] Cholesky factor of each diagonal block
-        double* Ldi;     // [kSparseMax][6] reciprocal of the factor's diagonal
-        double* y;       // [kSparseMax][6]
-        double* z;       // [kSparseMax][6]
-        double* x;       // [kSparseMax][6]
-        double* L;       // [cap][36] off-diagonal blocks, column by column
-        int cap;
-        // large teams only
-        uint32_t* radj;  // [kSpMax][kSpWords] row patterns, bit k = column eliminated k-th
+        int* rowptr;     // [n + 1] row lists: columns d with L(v, d) != 0
         int* deg;        // current degree of each node; later the level cursors
         int* sel;        // nodes eliminated in the current round
         int* lvl_work;   // largest column work of each level
+        int* rowidx;     // [kRowCapLarge]
         int* rowoff;     // [kRowCapLarge] block index of L(u, d) for each row-list entry
+        int* meta;       // [0] number of levels
+        double* Dg;      // [n][36] diagonal blocks
+        double* Ld;      // [n][36] Cholesky factor of each diagonal block
+        double* Ldi;     // [n][6] reciprocal of the factor's diagonal
+        double* y;       // [n][6]
+        double* z;       // [n][6]
+        double* x;       // [n][6]
+        double* L;       // [cap][36] off-diagonal blocks, column by column
+        int cap;
     };
     __device__ __forceinline__ Sparse sparse_ws() const {
-        if constexpr (kLargeTeam) {
-            constexpr int M = kSparseMaxLarge, M8 = kSparseMaxLarge + 8;
-            int* q = reinterpret_cast<int*>(B.sparse_big);
-            Sparse S;
-            S.adj = reinterpret_cast<uint32_t*>(q);
-            q += M * kSparseWordsLarge;
-            S.radj = reinterpret_cast<uint32_t*>(q);
-            q += M * kSparseWordsLarge;
-            S.perm = q; q += M8;
-            S.ipos = q; q += M8;
-            S.cstart = q; q += M8;
-            S.lvl_nodes = q; q += M8;
-            S.height = q; q += M8;
-            S.lvl_start = q; q += M8;
-            S.rowptr = q; q += M8;
-            S.deg = q; q += M8;
-            S.sel = q; q += M8;
-            S.lvl_work = q; q += M8;
-            q += 2 * M8;  // spare
-            S.rowidx = q; q += kRowCapLarge;
-            S.rowoff = q; q += kRowCapLarge;
-            S.meta = q;
-            double* d = B.sparse_big + (kSparseLargeIntWords + 1) / 2;
-            S.Dg = d; d += 36 * M;
-            S.Ld = d; d += 36 * M;
-            S.Ldi = d; d += 6 * M;
-            S.y = d; d += 6 * M;
-            S.z = d; d += 6 * M;
-            S.x = d; d += 6 * M;
-            S.L = d;
-            const long long left = B.sparse_big_doubles - kSparseLargeHeaderDoubles;
-            S.cap = left > 0 ? (int)min(left / 36, (long long)kRowCapLarge) : 0;
-            return S;
-        }
+        constexpr int M = kSparseMaxLarge, M8 = kSparseMaxLarge + 8;
+        int* q = reinterpret_cast<int*>(B.sparse_big);
+        Sparse S;
+        S.adj = reinterpret_cast<uint32_t*>(q);
+        q += M * kSparseWordsLarge;
+        S.radj = reinterpret_cast<uint32_t*>(q);
+        q += M * kSparseWordsLarge;
+        S.perm = q; q += M8;
+        S.ipos = q; q += M8;
+        S.cstart = q; q += M8;
+        S.lvl_nodes = q; q += M8;
+        S.height = q; q += M8;
+        S.lvl_start = q; q += M8;
+        S.rowptr = q; q += M8;
+        S.deg = q; q += M8;
+        S.sel = q; q += M8;
+        S.lvl_work = q; q += M8;
+        q += 2 * M8;  // spare
+        S.rowidx = q; q += kRowCapLarge;
+        S.rowoff = q; q += kRowCapLarge;
+        S.meta = q;
+        double* d = B.sparse_big + (kSparseLargeIntWords + 1) / 2;
+        S.Dg = d; d += 36 * M;
+        S.Ld = d; d += 36 * M;
+        S.Ldi = d; d += 6 * M;
+        S.y = d; d += 6 * M;
+        S.z = d; d += 6 * M;
+        S.x = d; d += 6 * M;
+        S.L = d;
+        const long long left = B.sparse_big_doubles - kSparseLargeHeaderDoubles;
+        S.cap = left > 0 ? (int)min(left / 36, (long long)kRowCapLarge) : 0;
+        return S;
+    }
+
+    // Scratch of the block and warp teams (one slot per team).  Everything is
+    // numbered by elimination position k (column k of the factor); the 6x6
+    // blocks of all columns lie in level order, column by column, each column's
+    // diagonal block first, so a block's index says what level it belongs to.
+    struct Direct {
+        uint32_t* adj;   // [kSparseMax][kSparseWords] node adjacency (thread blocks keep it in shared memory)
+        uint32_t* colb;  // [kSparseMax][kSparseWords] column k's pattern: positions u > k with L(u, k) != 0
+        uint32_t* rowb;  // [kSparseMax][kSparseWords] row k's pattern: positions d < k with L(k, d) != 0
+        int* perm;       // position -> node
+        int* ipos;       // node -> position
+        int* height;     // node -> elimination-tree height, then position -> height
+        int* deg;        // degree of each remaining node while ordering
+        int* body;       // position -> body
+        int* base;       // position -> index of the column's diagonal block
+        int* lvl_cols;   // positions by (height, position)
+        int* lvl_start;  // [levels + 1] first entry of each level in lvl_cols
+        int* lvl_blk;    // [levels + 1] first block of each level
+        int* lvl_len;    // [levels] longest update list of the level
+        int* meta;       // [0] levels, [1] blocks, [2] update-list entries
+        int* lbeg;       // [blocks + 1] start of each block's update list
+        unsigned short* ku;  // [blocks] (column << 8) | row of each block
+        double* Linv;    // [kSparseMax][kInvStride] packed inverse of each diagonal Cholesky factor
+        double* y;       // [kSparseMax][6] right-hand side, then L^-1 of it
+        double* x;       // [kSparseMax][6]
+        double* L;       // [cap][36] blocks
+        int cap;         // blocks
+    };
+    __device__ __forceinline__ Direct direct_ws() const {
         // thread-block teams use slot blockIdx.x of B.dense, warp teams slot
         // (T.slot - gridDim.x) of B.dense_warp
         const bool warp_slot = Team::kind == 1;
-        double* const base = warp_slot ? B.dense_warp + (long long)(T.slot - (int)gridDim.x) * B.dense_stride_warp
-                                       : B.dense + (long long)T.slot * B.dense_stride;
+        double* const first = warp_slot ? B.dense_warp + (long long)(T.slot - (int)gridDim.x) * B.dense_stride_warp
+                                        : B.dense + (long long)T.slot * B.dense_stride;
         const long long stride = warp_slot ? B.dense_stride_warp : B.dense_stride;
-        char* p = reinterpret_cast<char*>(base);
-        Sparse S;
-        S.adj = reinterpret_cast<uint32_t*>(p);
-        p += kSparseMax * kSparseWords * 4;
-        S.perm = reinterpret_cast<int*>(p);
-        p += kSparseMax * 4;
-        S.ipos = reinterpret_cast<int*>(p);
-        p += kSparseMax * 4;
-        S.cstart = reinterpret_cast<int*>(p);
-        p += (kSparseMax + 8) * 4;
-        S.lvl_nodes = reinterpret_cast<int*>(p);
-        p += kSparseMax * 4;
-        S.height = reinterpret_cast<int*>(p);
-        p += kSparseMax * 4;
-        S.lvl_start = reinterpret_cast<int*>(p);
-        p += (kSparseMax + 8) * 4;
-        S.rowptr = reinterpret_cast<int*>(p);
-        p += (kSparseMax + 8) * 4;
-        S.rowbase = reinterpret_cast<int*>(p);
-        p += (kSparseMax + 8) * 4;
-        S.lvl_mode = reinterpret_cast<int*>(p);
-        p += (kSparseMax + 8) * 4;
-        S.sub_start = reinterpret_cast<int*>(p);
-        p += (kSparseMax + 8) * 4;
-        S.sub_nodes = reinterpret_cast<int*>(p);
-        p += (kSparseMax + 8) * 4;
-        S.etp = reinterpret_cast<int*>(p);
-        p += (kSparseMax + 8) * 4;
-        S.swork = reinterpret_cast<int*>(p);
-        p += (kSparseMax + 8) * 4;
-        S.thr = reinterpret_cast<int*>(p);
-        p += (kSparseMax + 8) * 4;
-        S.rowidx = reinterpret_cast<int*>(p);
-        p += kRowCap * 4;
-        S.meta = reinterpret_cast<int*>(p);
-        p += 8 * 4;
-        S.Dg = reinterpret_cast<double*>(p);
-        p += kSparseMax * 36 * 8;
-        S.Ld = reinterpret_cast<double*>(p);
-        p += kSparseMax * 36 * 8;
-        S.Ldi = reinterpret_cast<double*>(p);
-        p += kSparseMax * 6 * 8;
-        S.y = reinterpret_cast<double*>(p);
-        p += kSparseMax * 6 * 8;
-        S.z = reinterpret_cast<double*>(p);
-        p += kSparseMax * 6 * 8;
-        S.x = reinterpret_cast<double*>(p);
-        p += kSparseMax * 6 * 8;
-        S.L = reinterpret_cast<double*>(p);
-        const long long used = (p - reinterpret_cast<char*>(base)) / 8;
-        S.cap = (int)((stride - used) / 36);
+        constexpr int M8 = kSparseMax + 8;
+        Direct S;
+        double* d = first;
+        S.Linv = d; d += kInvStride * kSparseMax;
+        S.y = d; d += 6 * kSparseMax;
+        S.x = d; d += 6 * kSparseMax;
+        int* q = reinterpret_cast<int*>(d);
+        S.colb = reinterpret_cast<uint32_t*>(q); q += kSparseMax * kSparseWords;
+        S.rowb = reinterpret_cast<uint32_t*>(q); q += kSparseMax * kSparseWords;
+        S.adj = reinterpret_cast<uint32_t*>(q); q += kSparseMax * kSparseWords;
+        S.perm = q; q += M8;
+        S.ipos = q; q += M8;
+        S.height = q; q += M8;
+        S.deg = q; q += M8;
+        S.body = q; q += M8;
+        S.base = q; q += M8;
+        S.lvl_cols = q; q += M8;
+        S.lvl_start = q; q += M8;
+        S.lvl_blk = q; q += M8;
+        S.lvl_len = q; q += M8;
+        S.meta = q; q += 8;
+        S.lbeg = q; q += kBlockCap + 8;
+        S.ku = reinterpret_cast<unsigned short*>(q);
+        S.L = first + (kSparseHeaderBytes + 255) / 256 * 32 - 36LL * kSparseMax;
+        S.cap = (int)((stride - (S.L - first)) / 36);
         return S;
     }
     // rank of node u among the set bits of a column pattern (= its block slot)
@@ -1220,29 +1215,22 @@ class SceneSolver {
         for (int k = 0; k < (u >> 5); ++k) r += __popc(w[k]);
         return r + __popc(w[u >> 5] & ((1u << (u & 31)) - 1u));
     }
-    // node of the a-th set bit of a column pattern
-    __device__ __forceinline__ static int bit_select(const uint32_t* w, int a) {
-        for (int k = 0; k < kSparseWords; ++k) {
-            const int c = __popc(w[k]);
-            if (a < c) {
-                uint32_t x = w[k];
-                for (int q = 0; q < a; ++q) x &= x - 1;
-                return (k << 5) + __ffs(x) - 1;
-            }
-            a -= c;
-        }
-        return -1;
-    }
-
-    // Symbolic factorisation, once per step: node adjacency from the incidence
-    // lists, greedy minimum-degree elimination on bitsets (ties to the smallest
-    // node), column patterns and block offsets.  Returns false (the scene then
-    // uses PCG) if the factor does not fit the scratch.
+    // Symbolic factorisation of the block and warp teams, once per step, every
+    // part spread over the team: node adjacency from the incidence lists, strict
+    // minimum-degree elimination on bitsets (ties to the smallest node), then --
+    // numbered by elimination position -- column and row patterns, levels of
+    // equal elimination-tree height, block storage in level order, and for every
+    // block its update list: the pairs of earlier blocks whose products it takes.
+    // The lists are what the numeric phase would otherwise look up bit by bit in
+    // every Newton iteration; they go behind the blocks, and a factor too dense
+    // to leave room for them (meta[2] = 0) walks the row patterns instead.
+    // Returns false (the scene then uses PCG) if the factor does not fit.
     __device__ bool sparse_symbolic() {
-        Sparse S = sparse_ws();
+        const Direct S = direct_ws();
+        constexpr int W = kSparseWords;
         const int n = n_active;
-        for (int q = tid; q < n * kSparseWords; q += nt) S.adj[q] = 0;
-        for (int q = tid; q < n; q += nt) S.ipos[q] = -1;
+        uint32_t* const adj = T.adjacency(S.adj);
+        for (int q = tid; q < n * W; q += nt) adj[q] = 0;
         T.sync();
         for (int l = tid; l < n_local; l += nt) {
             const int gb = B.lbody[b0 + l];
@@ -1250,178 +1238,180 @@ class SceneSolver {
             const int i = B.didx[gb];
             const int st0 = B.inc_start[gb], cnt = B.inc_cnt[gb];
             for (int k = 0; k < cnt; ++k) {
-                const int e = B.inc[st0 + k];
-                const int go = b0 + B.cbody[2 * (e >> 1) + (1 - (e & 1))];
-                if (go == gb || !active(go)) continue;
+                const int go = B.inc_o[st0 + k];  // -1: static
+                if (go == gb || go < 0 || !B.local[go]) continue;
                 const int j = B.didx[go];
-                S.adj[i * kSparseWords + (j >> 5)] |= 1u << (j & 31);
+                adj[i * W + (j >> 5)] |= 1u << (j & 31);
             }
+            int d = 0;
+            for (int w = 0; w < W; ++w) d += __popc(adj[i * W + w]);
+            S.deg[i] = d;
+            S.ipos[i] = -1;
+            S.height[i] = 0;
         }
         T.sync();
         for (int k = 0; k < n; ++k) {
             // argmin (degree, node) over the remaining nodes
-            double best[1] = {-1e300};
-            for (int i = tid; i < n; i += nt) {
-                if (S.ipos[i] >= 0) continue;
-                int d = 0;
-                for (int w = 0; w < kSparseWords; ++w) d += __popc(S.adj[i * kSparseWords + w]);
-                const double key = -(double)(d * 65536 + i);
-                best[0] = dmax(best[0], key);
-            }
-            T.max(best);
-            const int v = ((int)(-best[0])) & 65535;
-            const uint32_t* av = S.adj + v * kSparseWords;
+            unsigned best = 0xffffffffu;
+            for (int i = tid; i < n; i += nt)
+                if (S.ipos[i] < 0) best = min(best, ((unsigned)S.deg[i] << 16) | (unsigned)i);
+            const int v = (int)(T.min_u32(best) & 0xffffu);
+            const uint32_t* av = adj + v * W;
+            const int hv = S.height[v] + 1;
             for (int u = tid; u < n; u += nt) {
+                if (u == v) {
+                    S.perm[k] = v;
+                    S.ipos[v] = k;
+                    S.body[k] = B.dbody[b0 + v];
+                }
                 if (!((av[u >> 5] >> (u & 31)) & 1u)) continue;
-                uint32_t* au = S.adj + u * kSparseWords;
-                for (int w = 0; w < kSparseWords; ++w) au[w] |= av[w];
-                au[u >> 5] &= ~(1u << (u & 31));
-                au[v >> 5] &= ~(1u << (v & 31));
-            }
-            if (tid == 0) {
-                S.perm[k] = v;
-                S.ipos[v] = k;
-            }
-            T.sync();
+                uint32_t* au = adj + u * W;
+                int d = 0;
+                for (int w = 0; w < W; ++w) {
+                    uint32_t x = au[w] | av[w];
+                    if (w == (u >> 5)) x &= ~(1u << (u & 31));
+                    if (w == (v >> 5)) x &= ~(1u << (v & 31));
+                    au[w] = x;
+                    d += __popc(x);
+                }
+                S.deg[u] = d;
+                S.height[u] = max(S.height[u], hv);
+            }  // the next minimum's barrier orders these rows before their readers
         }
-        // block offsets in elimination order
-        if (tid == 0) {
-            int acc = 0;
-            for (int k = 0; k < n; ++k) {
-                const int v = S.perm[k];
-                S.cstart[v] = acc;
-                for (int w = 0; w < kSparseWords; ++w) acc += __popc(S.adj[v * kSparseWords + w]);
+        T.sync();
+        // patterns by position: word w of column k's and row k's pattern per item
+        for (int q = tid; q < n * W; q += nt) {
+            const int k = q / W, w = q - k * W;
+            const int v = S.perm[k];
+            uint32_t cb = 0, rb = 0;
+            const int end = min(n, 32 * w + 32);
+            for (int p = 32 * w; p < end; ++p) {
+                const int o = S.perm[p];
+                const uint32_t hit = p > k ? adj[v * W + (o >> 5)] >> (o & 31) : adj[o * W + (v >> 5)] >> (v & 31);
+                if (p > k) cb |= (hit & 1u) << (p & 31);
+                else if (p < k) rb |= (hit & 1u) << (p & 31);
             }
-            S.cstart[n] = acc;
-            if (acc <= S.cap && acc <= kRowCap) {
-                // row lists: for node u, the columns d (in elimination order)
-                // whose pattern contains u, i.e. the blocks L(u, d)
-                for (int v = 0; v <= n; ++v) S.rowptr[v] = 0;
-                for (int d = 0; d < n; ++d)
-                    for (int w = 0; w < kSparseWords; ++w) {
-                        uint32_t bits = S.adj[d * kSparseWords + w];
-                        while (bits) {
-                            S.rowptr[(w << 5) + __ffs(bits)]++;
-                            bits &= bits - 1;
-                        }
+            S.colb[q] = cb;
+            S.rowb[q] = rb;
+        }
+        for (int k = tid; k < n; k += nt) S.deg[k] = S.height[S.perm[k]];  // height by position
+        T.sync();
+        // position k's rank in (height, position) order and its first block: the
+        // sum over the columns before it of their block counts
+        for (int k = tid; k < n; k += nt) {
+            int m = 0;
+            for (int w = 0; w < W; ++w) m += __popc(S.colb[k * W + w]);
+            S.height[k] = m + 1;  // blocks of the column, from here on
+        }
+        T.sync();
+        int top = 0;
+        for (int k = tid; k < n; k += nt) {
+            const int h = S.deg[k];
+            int rank = 0, first = 0;
+            for (int j = 0; j < n; ++j) {
+                const int hj = S.deg[j];
+                if (hj < h || (hj == h && j < k)) {
+                    ++rank;
+                    first += S.height[j];
+                }
+            }
+            S.lvl_cols[rank] = k;
+            S.base[k] = first;
+            if (rank == n - 1) S.meta[1] = first + S.height[k];
+            top = max(top, h);
+        }
+        const int nlev = 0x7fffffff - (int)T.min_u32(0x7fffffffu - (unsigned)top) + 1;
+        for (int l = tid; l <= nlev; l += nt) {  // levels: columns and blocks of smaller height
+            int c = 0, b = 0;
+            for (int j = 0; j < n; ++j)
+                if (S.deg[j] < l) {
+                    ++c;
+                    b += S.height[j];
+                }
+            S.lvl_start[l] = c;
+            S.lvl_blk[l] = b;
+            S.lvl_len[l] = 0;
+        }
+        if (tid == 0) S.meta[0] = nlev;
+        T.sync();
+        const int nblk = S.meta[1];
+        if (nblk > S.cap) return false;
+        // (column, row) of every block
+        for (int q = tid; q < n * W; q += nt) {
+            const int k = q / W, w = q - k * W;
+            int b = S.base[k] + 1;
+            for (int x = 0; x < w; ++x) b += __popc(S.colb[k * W + x]);
+            uint32_t bits = S.colb[q];
+            while (bits) {
+                S.ku[b++] = (unsigned short)((k << 8) | ((w << 5) + __ffs(bits) - 1));
+                bits &= bits - 1;
+            }
+            if (w == 0) S.ku[S.base[k]] = (unsigned short)((k << 8) | k);
+        }
+        T.sync();
+        // update lists: block (u, k) takes L(u, d) L(k, d)^T for every d in the
+        // rows of both
+        T.scan(nblk, 0,
+               [&](int i) {
+                   const int k = S.ku[i] >> 8, u = S.ku[i] & 255;
+                   int c = 0;
+                   for (int w = 0; w < W; ++w) c += __popc(S.rowb[k * W + w] & S.rowb[u * W + w]);
+                   if (c) atomicMax(&S.lvl_len[S.deg[k]], c);
+                   return c;
+               },
+               [&](int i, int excl) {
+                   S.lbeg[i] = excl;
+                   if (i == nblk - 1) {
+                       const int k = S.ku[i] >> 8, u = S.ku[i] & 255;
+                       int c = 0;
+                       for (int w = 0; w < W; ++w) c += __popc(S.rowb[k * W + w] & S.rowb[u * W + w]);
+                       S.lbeg[nblk] = excl + c;
+                   }
+               });
+        T.sync();
+        const int total = S.lbeg[nblk];
+        const bool listed = total > 0 && (long long)total * 4 <= (long long)(S.cap - nblk) * 288;
+        if (tid == 0) S.meta[2] = listed ? total : 0;
+        if (listed) {
+            uint32_t* const list = reinterpret_cast<uint32_t*>(S.L + 36LL * nblk);
+            for (int i = tid; i < nblk; i += nt) {
+                const int k = S.ku[i] >> 8, u = S.ku[i] & 255;
+                int o = S.lbeg[i];
+                for (int w = 0; w < W; ++w) {
+                    uint32_t bits = S.rowb[k * W + w] & S.rowb[u * W + w];
+                    while (bits) {
+                        list[o++] = update_entry(S, k, u, (w << 5) + __ffs(bits) - 1);
+                        bits &= bits - 1;
                     }
-                for (int v = 0; v < n; ++v) S.rowptr[v + 1] += S.rowptr[v];
-                for (int v = 0; v < n; ++v) S.height[v] = S.rowptr[v];  // fill cursors
-                for (int k = 0; k < n; ++k) {
-                    const int d = S.perm[k];
-                    for (int w = 0; w < kSparseWords; ++w) {
-                        uint32_t bits = S.adj[d * kSparseWords + w];
-                        while (bits) {
-                            const int u = (w << 5) + __ffs(bits) - 1;
-                            bits &= bits - 1;
-                            S.rowidx[S.height[u]++] = d;
-                        }
-                    }
                 }
-                // elimination tree, column work (block products, the sum of the
-                // pattern sizes over the row list) and subtree work
-                for (int k = 0; k < n; ++k) {
-                    const int v = S.perm[k];
-                    int par = -1, best = n;
-                    for (int w = 0; w < kSparseWords; ++w) {
-                        uint32_t bits = S.adj[v * kSparseWords + w];
-                        while (bits) {
-                            const int u = (w << 5) + __ffs(bits) - 1;
-                            bits &= bits - 1;
-                            if (S.ipos[u] < best) { best = S.ipos[u]; par = u; }
-                        }
-                    }
-                    S.etp[v] = par;
-                    int work = 1;
-                    for (int q = S.rowptr[v]; q < S.rowptr[v + 1]; ++q) {
-                        const int d = S.rowidx[q];
-                        for (int w = 0; w < kSparseWords; ++w) work += __popc(S.adj[d * kSparseWords + w]);
-                    }
-                    S.height[v] = work;  // column work, for now
-                    S.swork[v] = 0;
+            }
+        }
+        // the block each incidence adds to: L(u, k) of its two bodies' positions,
+        // kept by the body eliminated first (-1: the other body keeps it, or the
+        // other body is static); inc_o is the PCG's and free here
+        for (int k = tid; k < n; k += nt) {
+            const int gb = S.body[k];
+            const int st0 = B.inc_start[gb], cnt = B.inc_cnt[gb];
+            for (int q = 0; q < cnt; ++q) {
+                const int go = B.inc_o[st0 + q];
+                int blk = -1;
+                if (go >= 0 && go != gb && B.local[go]) {
+                    const int u = S.ipos[B.didx[go]];
+                    if (u > k) blk = S.base[k] + 1 + bit_rank(S.colb + k * W, u);
                 }
-                for (int k = 0; k < n; ++k) {  // children before parents
-                    const int v = S.perm[k];
-                    S.swork[v] += S.height[v];
-                    if (S.etp[v] >= 0) S.swork[S.etp[v]] += S.swork[v];
-                }
-                // bottom subtrees (subtree work <= kSubWork) to threads; thr = -1
-                // above them.  The lanes of a warp whose subtrees take different
-                // paths run one after another, so each root goes to the warp with
-                // the least subtree work so far, on that warp's next lane
-                // (lvl_start holds the warps' work and root counts until the
-                // level pass below)
-                const int nwarp = nt >> 5;
-                int* wload = S.lvl_start;
-                int* wroots = S.lvl_start + 32;
-                for (int w = 0; w < nwarp; ++w) wload[w] = wroots[w] = 0;
-                for (int k = n - 1; k >= 0; --k) {  // parents before children
-                    const int v = S.perm[k], par = S.etp[v];
-                    if (S.swork[v] > kSubWork) {
-                        S.thr[v] = -1;
-                    } else if (par < 0 || S.thr[par] < 0) {
-                        int best = 0;
-                        for (int w = 1; w < nwarp; ++w)
-                            if (wload[w] < wload[best]) best = w;
-                        wload[best] += S.swork[v];
-                        S.thr[v] = 32 * best + (wroots[best]++ & 31);
-                    } else {
-                        S.thr[v] = S.thr[par];
-                    }
-                }
-                for (int t = 0; t <= nt; ++t) S.sub_start[t] = 0;
-                for (int v = 0; v < n; ++v)
-                    if (S.thr[v] >= 0) S.sub_start[S.thr[v] + 1]++;
-                for (int t = 0; t < nt; ++t) S.sub_start[t + 1] += S.sub_start[t];
-                for (int t = 0; t < nt; ++t) S.lvl_start[t] = S.sub_start[t];  // fill cursors
-                for (int k = 0; k < n; ++k) {
-                    const int v = S.perm[k];
-                    if (S.thr[v] >= 0) S.sub_nodes[S.lvl_start[S.thr[v]]++] = v;
-                }
-                // levels of the nodes above the bottom subtrees: a column can be
-                // factorised once every column that updates it is done; equal
-                // heights are independent
-                int nlev = 0, ntop = 0;
-                for (int k = 0; k < n; ++k) {
-                    const int v = S.perm[k];
-                    if (S.thr[v] >= 0) continue;
-                    const int work = S.height[v];
-                    int h = 0;
-                    for (int q = S.rowptr[v]; q < S.rowptr[v + 1]; ++q) {
-                        const int d = S.rowidx[q];
-                        if (S.thr[d] < 0) h = max(h, S.swork[d] + 1);  // swork of a top node: its height
-                    }
-                    S.swork[v] = h;
-                    S.height[v] = work;
-                    nlev = max(nlev, h + 1);
-                    ++ntop;
-                }
-                for (int l = 0; l <= nlev; ++l) S.lvl_start[l] = 0;
-                for (int v = 0; v < n; ++v)
-                    if (S.thr[v] < 0) S.lvl_start[S.swork[v] + 1]++;
-                for (int l = 0; l < nlev; ++l) S.lvl_start[l + 1] += S.lvl_start[l];
-                int pos = 0;  // stable in elimination order
-                for (int l = 0; l < nlev; ++l)
-                    for (int k = 0; k < n; ++k)
-                        if (S.thr[S.perm[k]] < 0 && S.swork[S.perm[k]] == l) S.lvl_nodes[pos++] = S.perm[k];
-                S.meta[0] = nlev;
-                // block rows of every top column (6 per pattern block + 6
-                // diagonal rows), in level order, and the fat levels
-                int rows = 0;
-                for (int l = 0; l < nlev; ++l) S.lvl_mode[l] = 0;
-                for (int q = 0; q < ntop; ++q) {
-                    const int v = S.lvl_nodes[q];
-                    int m = 0;
-                    for (int w = 0; w < kSparseWords; ++w) m += __popc(S.adj[v * kSparseWords + w]);
-                    S.rowbase[q] = rows;
-                    rows += 6 * (m + 1);
-                    if (S.height[v] - 1 > kFatWork) S.lvl_mode[S.swork[v]] = 1;
-                }
-                S.rowbase[ntop] = rows;
+                B.inc_o[st0 + q] = blk;
             }
         }
         T.sync();
-        return S.cstart[n] <= S.cap && S.cstart[n] <= kRowCap;
+        return true;
+    }
+    // Update-list entry of block (u, k) and column d: the block indices of L(u, d)
+    // and L(k, d); for the diagonal block (u = k) those of L(k, d) and of d itself,
+    // whose substitution vector the forward sweep takes.
+    __device__ __forceinline__ static uint32_t update_entry(const Direct& S, int k, int u, int d) {
+        const uint32_t* cd = S.colb + d * kSparseWords;
+        const uint32_t a = (uint32_t)(S.base[d] + 1 + bit_rank(cd, u));
+        return (a << 16) | (u == k ? (uint32_t)d : (uint32_t)(S.base[d] + 1 + bit_rank(cd, k)));
     }
 
     // Symbolic factorisation on the large-scene teams (up to kSparseMaxLarge
@@ -1641,7 +1631,7 @@ class SceneSolver {
         return depth[0] <= kDirectDepthMax;
     }
 
-    // Column block of active body gb: the diagonal block P and, per incidence
+    // Column block of active body gb (large-scene teams): the diagonal block P and, per incidence
     // with a body eliminated later, the off-diagonal block T_o K^-1 T_b^T
     // (linsysAddition's four blocks, :232-247).  Each column is owned by its
     // body's thread, so accumulation is race free and in incidence order.
@@ -1731,484 +1721,287 @@ class SceneSolver {
             x[i] = t * Li[i];
         }
     }
-    // C -= A B^T for 6x6 row-major blocks
-    __device__ __forceinline__ static void sub_abt6(double* Cm, const double* A, const double* Bm) {
-        for (int r = 0; r < 6; ++r) {
-            double a[6];
+    // Inverse of the lower Cholesky factor of a 6x6 SPD block (row-major, lower
+    // triangle read), packed by rows; false if not SPD.  One reciprocal square
+    // root per column is the whole chain: the diagonal of the factor itself is
+    // never needed.
+    __device__ __forceinline__ static bool chol6_inverse(const double* A, double* Li) {
+        double L[15], inv[6];  // strictly lower factor, packed by rows
 #pragma unroll
-            for (int q = 0; q < 6; ++q) a[q] = A[6 * r + q];
+        for (int j = 0; j < 6; ++j) {
+            double d = A[7 * j];
 #pragma unroll
-            for (int c = 0; c < 6; ++c) {
+            for (int k = 0; k < j; ++k) d -= L[j * (j - 1) / 2 + k] * L[j * (j - 1) / 2 + k];
+            if (!(d > 0.0)) return false;
+            inv[j] = rsqrt(d);
+#pragma unroll
+            for (int i = j + 1; i < 6; ++i) {
+                double t = A[6 * i + j];
+#pragma unroll
+                for (int k = 0; k < j; ++k) t -= L[i * (i - 1) / 2 + k] * L[j * (j - 1) / 2 + k];
+                L[i * (i - 1) / 2 + j] = t * inv[j];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+#pragma unroll
+            for (int j = 0; j < i; ++j) {
                 double t = 0.0;
 #pragma unroll
-                for (int q = 0; q < 6; ++q) t += a[q] * Bm[6 * c + q];
-                Cm[6 * r + c] -= t;
+                for (int k = j; k < i; ++k) t += L[i * (i - 1) / 2 + k] * Li[k * (k + 1) / 2 + j];
+                Li[i * (i + 1) / 2 + j] = -t * inv[i];
             }
+            Li[i * (i + 1) / 2 + i] = inv[i];
+        }
+        return true;
+    }
+    __device__ __forceinline__ static void ld6(const double* p, double* v) {  // 16-byte aligned
+        const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1],
+                      c = reinterpret_cast<const double2*>(p)[2];
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y;
+    }
+    __device__ __forceinline__ static void st6(double* p, const double* v) {
+        reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
+        reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
+        reinterpret_cast<double2*>(p)[2] = make_double2(v[4], v[5]);
+    }
+
+    // The Newton matrix and right-hand side of the block and warp teams' factor
+    // (linsysAddition's four blocks, :232-247), one thread per block row: row r of
+    // block (u, k) = T_u W T_k^T summed over the contacts of the two bodies in
+    // incidence order, T_j = s_j [I; C_j] with C_j = [c_j]x, i.e. from the 3x3
+    // blocks [W, W C_k^T; C_u W, C_u W C_k^T] with the sign of s_u s_k; a diagonal
+    // row takes every contact of the body, M / cm + eps I, and component r of
+    // rhs = sum T_j K^-1 sf - ru; rows of blocks that only fill in are zero.
+    __device__ void assemble_rows(double eps) const {
+        const Direct S = direct_ws();
+        const int rows = 6 * S.meta[1];
+        for (int t = tid; t < rows; t += nt) {
+            const int i = t / 6, r = t - 6 * i;
+            const int k = S.ku[i] >> 8, u = S.ku[i] & 255;
+            const int gb = S.body[k], st0 = B.inc_start[gb], cnt = B.inc_cnt[gb];
+            const bool diag = k == u;
+            double a[6] = {0, 0, 0, 0, 0, 0}, b = 0;
+            const int q3 = r < 3 ? r : r - 3;
+            for (int q = 0; q < cnt; ++q) {
+                if (!diag && B.inc_o[st0 + q] != i) continue;
+                const int e = B.inc[st0 + q], gc = e >> 1, side = e & 1;
+                const double* W = B.W + 6 * gc;
+                const d3 w0 = d3{W[0], W[3], W[4]}, w1 = d3{W[3], W[1], W[5]}, w2 = d3{W[4], W[5], W[2]};
+                const d3 ck = ld3(B.arm + 6 * gc + 3 * side);
+                const d3 cu = diag ? ck : ld3(B.arm + 6 * gc + 3 * (1 - side));
+                // row q3 of W, or of C_u W: (c x)_ab row q3 times W
+                d3 v;
+                if (r < 3) v = q3 == 0 ? w0 : (q3 == 1 ? w1 : w2);
+                else if (q3 == 0) v = sub3(scl3(cu.y, w2), scl3(cu.z, w1));
+                else if (q3 == 1) v = sub3(scl3(cu.z, w0), scl3(cu.x, w2));
+                else v = sub3(scl3(cu.x, w1), scl3(cu.y, w0));
+                const d3 z = cross3(ck, v);  // the row times C_k^T
+                if (diag) {
+                    a[0] += v.x; a[1] += v.y; a[2] += v.z; a[3] += z.x; a[4] += z.y; a[5] += z.z;
+                    const d3 x = ld3(B.Xi + 3LL * (st0 + q));
+                    const d3 h = r < 3 ? x : cross3(ck, x);
+                    b += q3 == 0 ? h.x : (q3 == 1 ? h.y : h.z);
+                } else {
+                    a[0] -= v.x; a[1] -= v.y; a[2] -= v.z; a[3] -= z.x; a[4] -= z.y; a[5] -= z.z;
+                }
+            }
+            if (diag) {
+                if (r < 3) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+                        if (c == r) a[c] += B.mass[gb] / cm + eps;
+                } else {
+                    const double* I = B.inertia + 6 * gb;
+                    const double ix = q3 == 0 ? I[0] : (q3 == 1 ? I[3] : I[4]);
+                    const double iy = q3 == 0 ? I[3] : (q3 == 1 ? I[1] : I[5]);
+                    const double iz = q3 == 0 ? I[4] : (q3 == 1 ? I[5] : I[2]);
+                    a[3] += ix / cm + (q3 == 0 ? eps : 0.0);
+                    a[4] += iy / cm + (q3 == 1 ? eps : 0.0);
+                    a[5] += iz / cm + (q3 == 2 ? eps : 0.0);
+                }
+                S.y[6 * k + r] = b - B.ru[6 * gb + r];
+            }
+            st6(S.L + 36LL * i + 6 * r, a);
         }
     }
 
-    // Fat level of the block team's factor: the level's block rows (6 per
-    // pattern block and 6 diagonal rows per column, numbered by S.rowbase) are
-    // spread over the team.  Row r of target block L(u, v) (or of the diagonal
-    // block) takes the updates of every column d of v's row list whose pattern
-    // holds u, in row-list order -- the same sums, in the same order, as the
-    // one-thread-per-column code; then each column's diagonal block is factored,
-    // then its rows are scaled by L_vv^-T.  A level with few rows (the top of
-    // the elimination tree: one column, a long row list) gives each row
-    // `split` (2, 4 or 8) adjacent lanes that take every split-th entry of the
-    // row list and combine their partial sums by an xor butterfly (every lane
-    // gets the same bits).
-    __device__ __forceinline__ int factor_level_rows(int l) {
-        const Sparse S = sparse_ws();
-        int bad = 0;
-        const int q0 = S.lvl_start[l], q1 = S.lvl_start[l + 1];
-        const int base = S.rowbase[q0], items = S.rowbase[q1] - base;
-        int split = 1;
-        while (split < 8 && items * split * 2 <= nt) split *= 2;
-        if (split > 1) {  // one round: items * split <= nt
-            const int it = tid / split, j = tid - it * split;
-            double part[6] = {0, 0, 0, 0, 0, 0};
-            double* dst = nullptr;
-            if (it < items) {
-                int lo = q0, hi = q1 - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (S.rowbase[mid] - base <= it) lo = mid;
-                    else hi = mid - 1;
-                }
-                const int v = S.lvl_nodes[lo];
-                const int loc = it - (S.rowbase[lo] - base);
-                const int a = loc / 6, r = loc - 6 * a;
-                const int m = (S.rowbase[lo + 1] - S.rowbase[lo]) / 6 - 1;
-                const bool diag = a == m;
-                const int u = diag ? v : bit_select(S.adj + v * kSpWords, a);
-                dst = diag ? S.Dg + 36 * v + 6 * r : S.L + 36LL * (S.cstart[v] + a) + 6 * r;
-                for (int k = S.rowptr[v] + j; k < S.rowptr[v + 1]; k += split) {
-                    const int d = S.rowidx[k];
-                    const uint32_t* ad = S.adj + d * kSpWords;
-                    if (!diag && !((ad[u >> 5] >> (u & 31)) & 1u)) continue;
-                    const double* Lvd = S.L + 36LL * (S.cstart[d] + bit_rank(ad, v));
-                    const double* Lud = diag ? Lvd : S.L + 36LL * (S.cstart[d] + bit_rank(ad, u));
-                    double x[6];
+    // One row's update by column d: acc -= x L^T with x = row r of L(u, d), L =
+    // L(k, d) (both 6x6); a diagonal row also takes its share of the forward
+    // substitution, x . y_d.
+    __device__ __forceinline__ static void row_update(const Direct& S, uint32_t e, bool diag, int r, double* acc,
+                                                      double& yr) {
+        const double* A = S.L + 36LL * (e >> 16);
+        const double* Bm = diag ? A : S.L + 36LL * (e & 0xffffu);
+        double x[6];
+        ld6(A + 6 * r, x);
 #pragma unroll
-                    for (int p = 0; p < 6; ++p) x[p] = Lud[6 * r + p];
+        for (int c = 0; c < 6; ++c) {
+            double b[6];
+            ld6(Bm + 6 * c, b);
+            double t = x[0] * b[0];
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) {
-                        double tt = 0.0;
-#pragma unroll
-                        for (int p = 0; p < 6; ++p) tt += x[p] * Lvd[6 * c + p];
-                        part[c] += tt;
-                    }
-                }
-            }
-            for (int o = 1; o < split; o <<= 1)
-#pragma unroll
-                for (int c = 0; c < 6; ++c) part[c] += __shfl_xor_sync(0xffffffffu, part[c], o);
-            if (dst && j == 0)
-                for (int c = 0; c < 6; ++c) dst[c] -= part[c];
+            for (int q = 1; q < 6; ++q) t += x[q] * b[q];
+            acc[c] -= t;
         }
-        for (int pass = split > 1 ? 1 : 0; pass < 2; ++pass) {
-            if (pass == 1) {  // diagonal blocks of the level, one thread per column
-                T.sync();
-                for (int q = q0 + tid; q < q1; q += nt) {
-                    const int v = S.lvl_nodes[q];
-                    double D[36], Lvv[36], Li[6];
-                    for (int e = 0; e < 36; ++e) D[e] = S.Dg[36 * v + e];
-                    if (!chol6(D, Lvv, Li)) {
-                        bad = 1;
-                        continue;
+        if (diag) {
+            double b[6];
+            ld6(S.y + 6 * (e & 0xffffu), b);
+            double t = x[0] * b[0];
+#pragma unroll
+            for (int q = 1; q < 6; ++q) t += x[q] * b[q];
+            yr -= t;
+        }
+    }
+
+    // Block Cholesky factorisation and both substitutions of the Newton system
+    // (block and warp teams; left-looking), one elimination-tree level at a time,
+    // the forward substitution riding along as one more component of each
+    // diagonal row.  Per level: (1) every row of the level's blocks takes its
+    // updates (the block's list of earlier blocks), a level with few rows giving
+    // each row 2 to 32 adjacent lanes that split the list and combine by an xor
+    // butterfly; (2) a thread per column inverts the Cholesky factor of its
+    // diagonal block and finishes its part of the forward substitution; (3) the
+    // other rows are scaled, A(u, k) L_kk^-T.  The backward substitution gives a
+    // column 8, 16 or 32 lanes (component x blocks) and no barrier but the
+    // level's.  Every scene of a batch spends most of its time here, bound by the
+    // chain of dependent loads of each level.  Looking up patterns bit by bit
+    // for every block product, one lane factoring and writing back a diagonal
+    // block, whole subtrees in sequence per warp and a separate forward sweep
+    // took 1,340 us per Newton iteration on a crate of 144 cubes and 49 us on a
+    // 10-box stack; this takes 750 and 32 us.  Stands in for the direct branch's
+    // SimplicialLDLT (:385-394).  Writes du; false on a non-SPD pivot, which only
+    // marks the scene: later columns then compute garbage in bounded loops.
+    __device__ bool direct_solve() {
+        const Direct S = direct_ws();
+        const int nlev = S.meta[0], nblk = S.meta[1];
+        const bool listed = S.meta[2] > 0;
+        const uint32_t* const list = reinterpret_cast<const uint32_t*>(S.L + 36LL * nblk);
+        bool bad = false;
+        for (int l = 0; l < nlev; ++l) {
+            const int q0 = S.lvl_start[l], q1 = S.lvl_start[l + 1];
+            const int i0 = S.lvl_blk[l], rows = 6 * (S.lvl_blk[l + 1] - i0), len = S.lvl_len[l];
+            if (len > 0) {
+                int split = 1;
+                if (listed)
+                    while (split < 32 && split < len && rows * split * 2 <= nt) split *= 2;
+                for (int t0 = 0; t0 < rows; t0 += nt) {  // split > 1: one round
+                    const int t = t0 + tid / split, j = tid & (split - 1);
+                    const bool on = t < rows;
+                    const int i = i0 + (on ? t : 0) / 6, r = on ? t - 6 * (i - i0) : 0;
+                    const int k = S.ku[i] >> 8, u = S.ku[i] & 255;
+                    const bool diag = k == u;
+                    double acc[6] = {0, 0, 0, 0, 0, 0}, yr = 0;
+                    if (on && j == 0) {
+                        ld6(S.L + 36LL * i + 6 * r, acc);
+                        if (diag) yr = S.y[6 * k + r];
                     }
-                    for (int e = 0; e < 36; ++e) S.Ld[36 * v + e] = Lvv[e];
-                    for (int e = 0; e < 6; ++e) S.Ldi[6 * v + e] = Li[e];
+                    if (on && listed) {
+                        for (int q = S.lbeg[i] + j; q < S.lbeg[i + 1]; q += split)
+                            row_update(S, list[q], diag, r, acc, yr);
+                    } else if (on) {
+                        for (int w = 0; w <= (k >> 5); ++w) {
+                            uint32_t bits = S.rowb[k * kSparseWords + w] & S.rowb[u * kSparseWords + w];
+                            while (bits) {
+                                row_update(S, update_entry(S, k, u, (w << 5) + __ffs(bits) - 1), diag, r, acc, yr);
+                                bits &= bits - 1;
+                            }
+                        }
+                    }
+                    for (int o = 1; o < split; o <<= 1) {
+#pragma unroll
+                        for (int c = 0; c < 6; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+                        yr += __shfl_xor_sync(0xffffffffu, yr, o);
+                    }
+                    if (on && j == 0) {
+                        st6(S.L + 36LL * i + 6 * r, acc);
+                        if (diag) S.y[6 * k + r] = yr;
+                    }
                 }
                 T.sync();
             }
-            for (int t = tid; t < items; t += nt) {
-                int lo = q0, hi = q1 - 1;  // the position q with rowbase[q] <= base + t < rowbase[q + 1]
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (S.rowbase[mid] - base <= t) lo = mid;
-                    else hi = mid - 1;
-                }
-                const int v = S.lvl_nodes[lo];
-                const int loc = t - (S.rowbase[lo] - base);
-                const int a = loc / 6, r = loc - 6 * a;
-                const int m = (S.rowbase[lo + 1] - S.rowbase[lo]) / 6 - 1;
-                const bool diag = a == m;
-                if (pass == 1) {
-                    if (diag) continue;
-                    double* row = S.L + 36LL * (S.cstart[v] + a) + 6 * r;
-                    double out[6];
-                    lsolve6(S.Ld + 36 * v, S.Ldi + 6 * v, row, out);
-                    for (int c = 0; c < 6; ++c) row[c] = out[c];
+            for (int q = q0 + tid; q < q1; q += nt) {
+                const int k = S.lvl_cols[q];
+                double Li[21], b[6];
+                if (!chol6_inverse(S.L + 36LL * S.base[k], Li)) {
+                    bad = true;
                     continue;
                 }
-                const uint32_t* av = S.adj + v * kSpWords;
-                const int u = diag ? v : bit_select(av, a);
-                double* dst = diag ? S.Dg + 36 * v + 6 * r : S.L + 36LL * (S.cstart[v] + a) + 6 * r;
-                double acc[6];
-                for (int c = 0; c < 6; ++c) acc[c] = dst[c];
-                for (int k = S.rowptr[v]; k < S.rowptr[v + 1]; ++k) {
-                    const int d = S.rowidx[k];
-                    const uint32_t* ad = S.adj + d * kSpWords;
-                    if (!diag && !((ad[u >> 5] >> (u & 31)) & 1u)) continue;
-                    const double* Lvd = S.L + 36LL * (S.cstart[d] + bit_rank(ad, v));
-                    const double* Lud = diag ? Lvd : S.L + 36LL * (S.cstart[d] + bit_rank(ad, u));
-                    double x[6];
+                ld6(S.y + 6 * k, b);
+                double* out = S.Linv + kInvStride * k;
 #pragma unroll
-                    for (int p = 0; p < 6; ++p) x[p] = Lud[6 * r + p];
+                for (int c = 0; c < 21; ++c) out[c] = Li[c];
+                double y[6];
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) {
-                        double tt = 0.0;
+                for (int r = 0; r < 6; ++r) {
+                    double t = 0.0;
 #pragma unroll
-                        for (int p = 0; p < 6; ++p) tt += x[p] * Lvd[6 * c + p];
-                        acc[c] -= tt;
+                    for (int c = 0; c <= r; ++c) t += Li[r * (r + 1) / 2 + c] * b[c];
+                    y[r] = t;
+                }
+                st6(S.y + 6 * k, y);
+            }
+            T.sync();
+            if (rows == 6 * (q1 - q0)) continue;  // no off-diagonal block in this level
+            for (int t = tid; t < rows; t += nt) {
+                const int i = i0 + t / 6, r = t - 6 * (i - i0);
+                const int k = S.ku[i] >> 8;
+                if ((S.ku[i] & 255) == k) continue;
+                double* row = S.L + 36LL * i + 6 * r;
+                const double* Li = S.Linv + kInvStride * k;
+                double a[6], o[6];
+                ld6(row, a);
+#pragma unroll
+                for (int c = 0; c < 6; ++c) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int q = 0; q <= c; ++q) s += a[q] * Li[c * (c + 1) / 2 + q];
+                    o[c] = s;
+                }
+                st6(row, o);
+            }
+            T.sync();
+        }
+        if (T.any(bad)) return false;
+        const int c = min(tid & 7, 5), cc = tid & 7;
+        for (int l = nlev - 1; l >= 0; --l) {
+            const int q0 = S.lvl_start[l], ncol = S.lvl_start[l + 1] - q0;
+            int sub = 1;  // groups of 8 lanes per column
+            while (sub < 4 && ncol * 16 * sub <= nt) sub *= 2;
+            const int ng = nt / (8 * sub), grp = tid / (8 * sub), j = (tid >> 3) & (sub - 1);
+            for (int g0 = 0; g0 < ncol; g0 += ng) {
+                const bool on = g0 + grp < ncol;
+                const int k = S.lvl_cols[q0 + (on ? g0 + grp : 0)];
+                const int blk = S.base[k];
+                double s = 0.0;
+                if (on) {
+                    int m = 0;
+                    for (int w = k >> 5; w < kSparseWords; ++w) m += __popc(S.colb[k * kSparseWords + w]);
+                    for (int a = 1 + j; a <= m; a += sub) {
+                        const double* Lb = S.L + 36LL * (blk + a) + c;
+                        double x[6];
+                        ld6(S.x + 6 * (S.ku[blk + a] & 255), x);
+#pragma unroll
+                        for (int r = 0; r < 6; ++r) s += Lb[6 * r] * x[r];
                     }
                 }
-                for (int c = 0; c < 6; ++c) dst[c] = acc[c];
-            }
-        }
-        return bad;
-    }
-
-    // Forward substitution of a fat level: a warp per column, the lanes
-    // splitting the column's row list, partials summed by a fixed shuffle tree.
-    __device__ __forceinline__ void forward_level_warp(int l) {
-        const Sparse S = sparse_ws();
-        const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
-        for (int q = S.lvl_start[l] + warp; q < S.lvl_start[l + 1]; q += nwarp) {
-            const int v = S.lvl_nodes[q];
-            double s6[6] = {0, 0, 0, 0, 0, 0};
-            for (int k = S.rowptr[v] + lane; k < S.rowptr[v + 1]; k += 32) {
-                const int d = S.rowidx[k];
-                const double* Lvd = S.L + 36LL * (S.cstart[d] + bit_rank(S.adj + d * kSpWords, v));
-                const double* yd = S.y + 6 * d;
-                for (int i = 0; i < 6; ++i) {
-                    double t = 0.0;
-                    for (int c = 0; c < 6; ++c) t += Lvd[6 * i + c] * yd[c];
-                    s6[i] += t;
-                }
-            }
-            warp_sum6(s6);
-            if (lane == 0) {
-                const int gb = B.dbody[b0 + v];
-                double b6[6], yv[6];
-                for (int r = 0; r < 6; ++r) b6[r] = B.rhs[6 * gb + r] - s6[r];
-                lsolve6(S.Ld + 36 * v, S.Ldi + 6 * v, b6, yv);
-                for (int r = 0; r < 6; ++r) S.y[6 * v + r] = yv[r];
-            }
-        }
-    }
-    // Backward substitution of a fat level: a warp per column, the lanes
-    // splitting the column's pattern blocks.
-    __device__ __forceinline__ void backward_level_warp(int l) {
-        const Sparse S = sparse_ws();
-        const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
-        for (int q = S.lvl_start[l] + warp; q < S.lvl_start[l + 1]; q += nwarp) {
-            const int v = S.lvl_nodes[q];
-            const uint32_t* av = S.adj + v * kSpWords;
-            const double* colv = S.L + 36LL * S.cstart[v];
-            const int m = (S.rowbase[q + 1] - S.rowbase[q]) / 6 - 1;
-            double s6[6] = {0, 0, 0, 0, 0, 0};
-            for (int a = lane; a < m; a += 32) {
-                const int u = bit_select(av, a);
-                const double* blk = colv + 36 * a;
-                const double* xu = S.x + 6 * u;
-                for (int c = 0; c < 6; ++c) {
-                    double t = 0.0;
-                    for (int r = 0; r < 6; ++r) t += blk[6 * r + c] * xu[r];
-                    s6[c] += t;
-                }
-            }
-            warp_sum6(s6);
-            if (lane == 0) {
-                double r6[6], xv[6];
-                for (int r = 0; r < 6; ++r) r6[r] = S.y[6 * v + r] - s6[r];
-                ltsolve6(S.Ld + 36 * v, S.Ldi + 6 * v, r6, xv);
-                for (int r = 0; r < 6; ++r) S.x[6 * v + r] = xv[r];
-                const int gb = B.dbody[b0 + v];
-                for (int r = 0; r < 6; ++r) B.du[6 * gb + r] = xv[r];
-            }
-        }
-    }
-
-    // One column of the factor by one thread (left-looking): D = A_vv - sum
-    // L(v,d) L(v,d)^T and L(u,v) -= L(u,d) L(v,d)^T over the columns d of v's
-    // row list, then L_vv = chol(D) and L(u,v) = A(u,v) L_vv^-T.  Returns 1 on a
-    // non-SPD pivot (the column is left unscaled).
-    __device__ __forceinline__ int factor_column(const Sparse& S, int v) const {
-        const uint32_t* av = S.adj + v * kSpWords;
-        double* colv = S.L + 36LL * S.cstart[v];
-        double D[36];
-        for (int e = 0; e < 36; ++e) D[e] = S.Dg[36 * v + e];
-        for (int r = S.rowptr[v]; r < S.rowptr[v + 1]; ++r) {
-            const int d = S.rowidx[r];
-            const uint32_t* ad = S.adj + d * kSpWords;
-            const double* cold = S.L + 36LL * S.cstart[d];
-            const double* Lvd = cold + 36 * bit_rank(ad, v);
-            sub_abt6(D, Lvd, Lvd);
-            int a = 0;  // walk pattern(d): u after v -> L(u,v) -= L(u,d) L(v,d)^T
-            for (int w = 0; w < spw(); ++w) {
-                uint32_t bits = ad[w];
-                while (bits) {
-                    const int u = (w << 5) + __ffs(bits) - 1;
-                    bits &= bits - 1;
-                    if (u != v && S.ipos[u] > S.ipos[v]) sub_abt6(colv + 36 * bit_rank(av, u), cold + 36 * a, Lvd);
-                    ++a;
-                }
-            }
-        }
-        double Lvv[36], Li[6];
-        if (!chol6(D, Lvv, Li)) return 1;
-        for (int e = 0; e < 36; ++e) S.Ld[36 * v + e] = Lvv[e];
-        for (int e = 0; e < 6; ++e) S.Ldi[6 * v + e] = Li[e];
-        int m = 0;
-        for (int w = 0; w < spw(); ++w) m += __popc(av[w]);
-        for (int a = 0; a < m; ++a) {  // L(u,v) = A(u,v) L_vv^-T, row by row
-            double* blk = colv + 36 * a;
-            for (int r = 0; r < 6; ++r) {
-                double row[6];
-                lsolve6(Lvv, Li, blk + 6 * r, row);
-                for (int c = 0; c < 6; ++c) blk[6 * r + c] = row[c];
-            }
-        }
-        return 0;
-    }
-    // One column of the factor by one warp: the column's block rows (6 per
-    // pattern block, 6 for the diagonal block) over the lanes, each summing the
-    // updates of v's row list in row-list order (the sums of factor_column);
-    // lane 0 factors the diagonal block, the lanes scale the rows by L_vv^-T.
-    // Every lane returns 1 on a non-SPD pivot.
-    __device__ __forceinline__ int factor_column_warp(const Sparse& S, int v, int lane) const {
-        const uint32_t* av = S.adj + v * kSpWords;
-        int m = 0;
-        for (int w = 0; w < spw(); ++w) m += __popc(av[w]);
-        for (int t = lane; t < 6 * (m + 1); t += 32) {
-            const int a = t / 6, r = t - 6 * a;
-            const bool diag = a == m;
-            const int u = diag ? v : bit_select(av, a);
-            double* dst = diag ? S.Dg + 36 * v + 6 * r : S.L + 36LL * (S.cstart[v] + a) + 6 * r;
-            double acc[6];
-            for (int c = 0; c < 6; ++c) acc[c] = dst[c];
-            for (int k = S.rowptr[v]; k < S.rowptr[v + 1]; ++k) {
-                const int d = S.rowidx[k];
-                const uint32_t* ad = S.adj + d * kSpWords;
-                if (!diag && !((ad[u >> 5] >> (u & 31)) & 1u)) continue;
-                const double* Lvd = S.L + 36LL * (S.cstart[d] + bit_rank(ad, v));
-                const double* Lud = diag ? Lvd : S.L + 36LL * (S.cstart[d] + bit_rank(ad, u));
-                double x[6];
+                for (int o = 8; o < 8 * sub; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                const double r = S.y[6 * k + c] - s;
+                const double* Li = S.Linv + kInvStride * k;
+                double x = 0.0;
 #pragma unroll
-                for (int p = 0; p < 6; ++p) x[p] = Lud[6 * r + p];
-#pragma unroll
-                for (int c = 0; c < 6; ++c) {
-                    double tt = 0.0;
-#pragma unroll
-                    for (int p = 0; p < 6; ++p) tt += x[p] * Lvd[6 * c + p];
-                    acc[c] -= tt;
+                for (int p = 0; p < 6; ++p) {
+                    const double rp = __shfl_sync(0xffffffffu, r, p, 8);
+                    if (p >= c) x += Li[p * (p + 1) / 2 + c] * rp;
+                }
+                if (on && j == 0 && cc < 6) {
+                    S.x[6 * k + cc] = x;
+                    B.du[6 * S.body[k] + cc] = x;
                 }
             }
-            for (int c = 0; c < 6; ++c) dst[c] = acc[c];
-        }
-        __syncwarp();
-        int bad = 0;
-        if (lane == 0) {
-            double D[36], Lvv[36], Li[6];
-            for (int e = 0; e < 36; ++e) D[e] = S.Dg[36 * v + e];
-            if (chol6(D, Lvv, Li)) {
-                for (int e = 0; e < 36; ++e) S.Ld[36 * v + e] = Lvv[e];
-                for (int e = 0; e < 6; ++e) S.Ldi[6 * v + e] = Li[e];
-            } else {
-                bad = 1;
-            }
-        }
-        bad = __shfl_sync(0xffffffffu, bad, 0);
-        __syncwarp();
-        if (!bad)
-            for (int t = lane; t < 6 * m; t += 32) {
-                double* row = S.L + 36LL * S.cstart[v] + 6 * t;  // block t / 6, row t % 6
-                double out[6];
-                lsolve6(S.Ld + 36 * v, S.Ldi + 6 * v, row, out);
-                for (int c = 0; c < 6; ++c) row[c] = out[c];
-            }
-        __syncwarp();
-        return bad;
-    }
-    // Forward and backward substitution of one column by one warp: lanes 6e + i
-    // (e < 5) take the row-list entry (pattern block) e of a round of five and
-    // row i; lane i then subtracts the round's products in entry order, so each
-    // component sees the same operations in the same order as forward_column /
-    // backward_column; lane 0 applies the diagonal block.
-    __device__ __forceinline__ void forward_column_warp(const Sparse& S, int v, int lane) const {
-        const int gb = B.dbody[b0 + v];
-        const int k0 = S.rowptr[v], k1 = S.rowptr[v + 1];
-        const int e = lane / 6, i = lane - 6 * e;
-        double b = lane < 6 ? B.rhs[6 * gb + lane] : 0.0;
-        for (int kb = k0; kb < k1; kb += 5) {
-            double t = 0.0;
-            if (e < 5 && kb + e < k1) {
-                const int d = S.rowidx[kb + e];
-                const double* Lvd = S.L + 36LL * (S.cstart[d] + bit_rank(S.adj + d * kSpWords, v));
-                const double* yd = S.y + 6 * d;
-                for (int c = 0; c < 6; ++c) t += Lvd[6 * i + c] * yd[c];
-            }
-            for (int q = 0; q < 5; ++q) {
-                const double tq = __shfl_sync(0xffffffffu, t, 6 * q + i);
-                if (lane < 6 && kb + q < k1) b -= tq;
-            }
-        }
-        double b6[6];
-        for (int r = 0; r < 6; ++r) b6[r] = __shfl_sync(0xffffffffu, b, r);
-        if (lane == 0) {
-            double yv[6];
-            lsolve6(S.Ld + 36 * v, S.Ldi + 6 * v, b6, yv);
-            for (int r = 0; r < 6; ++r) S.y[6 * v + r] = yv[r];
-        }
-        __syncwarp();
-    }
-    __device__ __forceinline__ void backward_column_warp(const Sparse& S, int v, int lane) const {
-        const uint32_t* av = S.adj + v * kSpWords;
-        const double* colv = S.L + 36LL * S.cstart[v];
-        int m = 0;
-        for (int w = 0; w < spw(); ++w) m += __popc(av[w]);
-        const int e = lane / 6, c = lane - 6 * e;
-        double r = lane < 6 ? S.y[6 * v + lane] : 0.0;
-        for (int ab = 0; ab < m; ab += 5) {
-            double t = 0.0;
-            if (e < 5 && ab + e < m) {
-                const double* blk = colv + 36 * (ab + e);
-                const double* xu = S.x + 6 * bit_select(av, ab + e);
-                for (int rr = 0; rr < 6; ++rr) t += blk[6 * rr + c] * xu[rr];
-            }
-            for (int q = 0; q < 5; ++q) {
-                const double tq = __shfl_sync(0xffffffffu, t, 6 * q + c);
-                if (lane < 6 && ab + q < m) r -= tq;
-            }
-        }
-        double r6[6];
-        for (int k = 0; k < 6; ++k) r6[k] = __shfl_sync(0xffffffffu, r, k);
-        if (lane == 0) {
-            double xv[6];
-            ltsolve6(S.Ld + 36 * v, S.Ldi + 6 * v, r6, xv);
-            for (int k = 0; k < 6; ++k) S.x[6 * v + k] = xv[k];
-            const int gb = B.dbody[b0 + v];
-            for (int k = 0; k < 6; ++k) B.du[6 * gb + k] = xv[k];
-        }
-        __syncwarp();
-    }
-    // forward substitution of one column: y_v = L_vv^-1 (b_v - sum L(v,d) y_d)
-    __device__ __forceinline__ void forward_column(const Sparse& S, int v) const {
-        const int gb = B.dbody[b0 + v];
-        double b6[6], yv[6];
-        for (int r = 0; r < 6; ++r) b6[r] = B.rhs[6 * gb + r];
-        for (int r = S.rowptr[v]; r < S.rowptr[v + 1]; ++r) {
-            const int d = S.rowidx[r];
-            const double* Lvd = S.L + 36LL * (S.cstart[d] + bit_rank(S.adj + d * kSpWords, v));
-            const double* yd = S.y + 6 * d;
-            for (int i = 0; i < 6; ++i) {
-                double t = 0.0;
-                for (int c = 0; c < 6; ++c) t += Lvd[6 * i + c] * yd[c];
-                b6[i] -= t;
-            }
-        }
-        lsolve6(S.Ld + 36 * v, S.Ldi + 6 * v, b6, yv);
-        for (int r = 0; r < 6; ++r) S.y[6 * v + r] = yv[r];
-    }
-    // backward substitution of one column: x_v = L_vv^-T (y_v - sum L(u,v)^T x_u)
-    __device__ __forceinline__ void backward_column(const Sparse& S, int v) const {
-        const uint32_t* av = S.adj + v * kSpWords;
-        const double* colv = S.L + 36LL * S.cstart[v];
-        double r6[6], xv[6];
-        for (int r = 0; r < 6; ++r) r6[r] = S.y[6 * v + r];
-        int a = 0;
-        for (int w = 0; w < spw(); ++w) {
-            uint32_t bits = av[w];
-            while (bits) {
-                const int u = (w << 5) + __ffs(bits) - 1;
-                bits &= bits - 1;
-                const double* blk = colv + 36 * a;
-                const double* xu = S.x + 6 * u;
-                for (int c = 0; c < 6; ++c) {
-                    double t = 0.0;
-                    for (int r = 0; r < 6; ++r) t += blk[6 * r + c] * xu[r];
-                    r6[c] -= t;
-                }
-                ++a;
-            }
-        }
-        ltsolve6(S.Ld + 36 * v, S.Ldi + 6 * v, r6, xv);
-        for (int r = 0; r < 6; ++r) S.x[6 * v + r] = xv[r];
-        const int gb = B.dbody[b0 + v];
-        for (int r = 0; r < 6; ++r) B.du[6 * gb + r] = xv[r];
-    }
-
-    // Block Cholesky factorisation + solve of the Newton system (left-looking).
-    // The bottom subtrees of the elimination tree (a stack of boxes is one such
-    // chain) belong to threads, balanced over the warps; a warp factors its
-    // lanes' subtrees column by column (factor_column_warp) and each thread
-    // sweeps its own, in elimination order, with no team barrier; the columns
-    // above them go one elimination-tree level at
-    // a time (columns of a level are independent): a thin level a warp per
-    // column when it has at most one column per warp, else a thread per column,
-    // a fat one its block rows over the team (factor_level_rows).  A
-    // non-SPD pivot only marks the scene, read once after the factorisation;
-    // later columns then compute garbage in bounded loops.  Stands in for the
-    // direct branch's SimplicialLDLT (:385-394).  Writes du; false on a non-SPD
-    // pivot.
-    __device__ bool dense_solve() {
-        if constexpr (kLargeTeam) return dense_solve_warp();
-        Sparse S = sparse_ws();
-        const int nlev = S.meta[0];
-        const int lane = tid & 31, w0 = tid - lane;
-        int bad = 0;
-        {  // each warp factors its lanes' subtrees, lane by lane, a warp per column
-            for (int ln = 0; ln < 32; ++ln)
-                for (int q = S.sub_start[w0 + ln]; q < S.sub_start[w0 + ln + 1]; ++q)
-                    bad |= factor_column_warp(S, S.sub_nodes[q], lane);
-        }
-        T.sync();
-        for (int l = 0; l < nlev; ++l) {
-            const int lq0 = S.lvl_start[l], ncol = S.lvl_start[l + 1] - lq0;
-            if (S.lvl_mode[l]) bad |= factor_level_rows(l);
-            else if (ncol <= (nt >> 5)) {  // few columns: a warp per column
-                if ((tid >> 5) < ncol) bad |= factor_column_warp(S, S.lvl_nodes[lq0 + (tid >> 5)], lane);
-            } else
-                for (int q = lq0 + tid; q < lq0 + ncol; q += nt) bad |= factor_column(S, S.lvl_nodes[q]);
-            T.sync();  // level barrier; a failed pivot is checked once after the factorisation
-        }
-        {
-            double fl[1] = {(double)bad};
-            T.max(fl);
-            bad = fl[0] > 0;
-        }
-        if (!bad) {
-            for (int ln = 0; ln < 32; ++ln)
-                for (int q = S.sub_start[w0 + ln]; q < S.sub_start[w0 + ln + 1]; ++q)
-                    forward_column_warp(S, S.sub_nodes[q], lane);
             T.sync();
-            for (int l = 0; l < nlev; ++l) {
-                const int lq0 = S.lvl_start[l], ncol = S.lvl_start[l + 1] - lq0;
-                if (S.lvl_mode[l]) forward_level_warp(l);
-                else if (ncol <= (nt >> 5)) {
-                    if ((tid >> 5) < ncol) forward_column_warp(S, S.lvl_nodes[lq0 + (tid >> 5)], lane);
-                } else
-                    for (int q = lq0 + tid; q < lq0 + ncol; q += nt) forward_column(S, S.lvl_nodes[q]);
-                T.sync();
-            }
-            for (int l = nlev - 1; l >= 0; --l) {
-                const int lq0 = S.lvl_start[l], ncol = S.lvl_start[l + 1] - lq0;
-                if (S.lvl_mode[l]) backward_level_warp(l);
-                else if (ncol <= (nt >> 5)) {
-                    if ((tid >> 5) < ncol) backward_column_warp(S, S.lvl_nodes[lq0 + (tid >> 5)], lane);
-                } else
-                    for (int q = lq0 + tid; q < lq0 + ncol; q += nt) backward_column(S, S.lvl_nodes[q]);
-                T.sync();
-            }
-            for (int ln = 0; ln < 32; ++ln)
-                for (int q = S.sub_start[w0 + ln + 1] - 1; q >= S.sub_start[w0 + ln]; --q)
-                    backward_column_warp(S, S.sub_nodes[q], lane);
         }
-        T.sync();
-        return !bad;
+        return true;
     }
 
     // node of the a-th set bit among the first nw words of a pattern
@@ -2950,7 +2743,8 @@ class SceneSolver {
         st.char_mass = cm;
         st.char_speed = cs;
         st.n_local_bodies = n_local;
-        st.factor_blocks = dense_mode ? sparse_ws().cstart[n_active] : 0;
+        if constexpr (kLargeTeam) st.factor_blocks = dense_mode ? sparse_ws().cstart[n_active] : 0;
+        else st.factor_blocks = dense_mode ? direct_ws().meta[1] - n_active : 0;
         st.team = Team::kind;
         st.status = status;
     }
@@ -3071,9 +2865,10 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) solve_scenes_kernel(co
                                                            const __grid_constant__ EngineCfg C) {
     __shared__ double s_red[2 * 16 * 32];
     __shared__ int s_int[33];
+    __shared__ uint32_t s_adj[kSparseMax * kSparseWords];
     __shared__ int s_q;
     {
-        CtaTeam T(s_red, s_int);
+        CtaTeam T(s_red, s_int, s_adj);
         const int n_cta = B.counts[0];
         for (;;) {
             if (threadIdx.x == 0) s_q = atomicAdd(&B.counts[2], 1);
