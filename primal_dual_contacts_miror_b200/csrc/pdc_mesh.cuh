@@ -7,21 +7,26 @@
 // signed distance (libigl, pseudonormal sign) and keeps the vertices inside:
 // position = the vertex, depth = -distance, normal = the other mesh's vertex
 // normals interpolated at the closest point, from the lower body to the
-// higher.  Here, per pair of meshes:
-//   1. mesh_pairs_kernel: every triangle pair whose world AABBs overlap gets a
+// higher.  Here, for all pairs of a query at once (one launch each):
+//   1. mesh_world_kernel: world vertices and box of both meshes;
+//   2. mesh_cull_kernel: the triangles of either mesh that meet the other's box;
+//   3. mesh_pairs_kernel: every pair of those whose boxes overlap gets a
 //      separating-axis test (both normals, nine edge-edge cross products, six
-//      in-plane edge normals; closed triangles); overlapping pairs flag both
-//      triangles (the seeds);
-//   2. mesh_sdf_kernel: one warp per vertex of a flagged triangle, the lanes
-//      splitting the other mesh's triangles (closest point by Voronoi regions,
-//      Ericson 5.1.5), the closest triangle the first of least squared
-//      distance (a fixed-order warp reduction), the sign from the
-//      angle-weighted pseudonormal of the closest feature (Baerentzen and
-//      Aanaes 2005): face, edge or vertex by which barycentric coordinates are
-//      below 1e-12;
-//   3. mesh_merge_kernel: the inside vertices, the first mesh's in index order
+//      in-plane edge normals; closed triangles); the vertices of overlapping
+//      pairs are the seeds;
+//   4. mesh_sdf_kernel: one warp per seed, the lanes splitting the other mesh's
+//      triangles (closest point by Voronoi regions, Ericson 5.1.5), the closest
+//      triangle the first of least squared distance (a fixed-order warp
+//      reduction), the sign from the angle-weighted pseudonormal of the closest
+//      feature (Baerentzen and Aanaes 2005): face, edge or vertex by which
+//      barycentric coordinates are below 1e-12;
+//   5. mesh_merge_kernel: the inside vertices, the first mesh's in index order
 //      then the second's, sorted and merged as every pair's points are
 //      (merge_points), frames and lever arms.
+// Testing every triangle pair of the two meshes (transforming both triangles
+// each time), six launches per pair and one thread merging took 7.5 ms for the 31
+// pairs of a chain of 1,140-triangle links; what is left is bound by launches,
+// the allocation and the copies.
 // The reference's breadth-first growth from the seed vertices walks an
 // adjacency map holding triangle-local corner numbers (Mesh.cpp:66-74), so it
 // can only revisit vertices 0-2; the seed vertices alone are kept here.
@@ -128,59 +133,148 @@ __device__ inline bool tri_separated(const d3* P, const d3* Q) {
     return false;
 }
 
-// Triangle pairs (i of A, j of B) whose world AABBs overlap and that no axis
-// separates: both triangles flagged (identical racing stores of 1).
-__global__ void __launch_bounds__(256) mesh_pairs_kernel(const MeshDev A, const MeshDev B, int* flag_a,
-                                                         int* flag_b) {
-    const long long total = (long long)A.nf * B.nf;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total; q += stride) {
-        const int i = (int)(q / B.nf), j = (int)(q - (long long)i * B.nf);
-        d3 P[3], Q[3];
-        for (int k = 0; k < 3; ++k) {
-            P[k] = world_vertex(A, A.F[3 * i + k]);
-            Q[k] = world_vertex(B, B.F[3 * j + k]);
-        }
-        const double pl[3] = {fmin(fmin(P[0].x, P[1].x), P[2].x), fmin(fmin(P[0].y, P[1].y), P[2].y),
-                              fmin(fmin(P[0].z, P[1].z), P[2].z)};
-        const double ph[3] = {fmax(fmax(P[0].x, P[1].x), P[2].x), fmax(fmax(P[0].y, P[1].y), P[2].y),
-                              fmax(fmax(P[0].z, P[1].z), P[2].z)};
-        const double ql[3] = {fmin(fmin(Q[0].x, Q[1].x), Q[2].x), fmin(fmin(Q[0].y, Q[1].y), Q[2].y),
-                              fmin(fmin(Q[0].z, Q[1].z), Q[2].z)};
-        const double qh[3] = {fmax(fmax(Q[0].x, Q[1].x), Q[2].x), fmax(fmax(Q[0].y, Q[1].y), Q[2].y),
-                              fmax(fmax(Q[0].z, Q[1].z), Q[2].z)};
-        if (ph[0] < ql[0] || qh[0] < pl[0] || ph[1] < ql[1] || qh[1] < pl[1] || ph[2] < ql[2] || qh[2] < pl[2])
-            continue;
-        if (!tri_separated(P, Q)) {
-            flag_a[i] = 1;
-            flag_b[j] = 1;
+// One mesh pair of a query: both meshes, and where its part of the scratch
+// begins (ints, doubles, output rows).
+struct MeshPair {
+    MeshDev m[2];
+    long long i0;    // zeroed ints: 8 counters, triangle flags of both, seed and inside flags of all vertices
+    long long j0;    // other ints: candidate triangles of both, seeds of both, order of the inside vertices
+    long long d0;    // doubles: 12 of boxes, then per vertex world position, contact position, normal, depth
+    long long row0;  // first row of the pair's merged contacts
+};
+struct MeshScratch {
+    const MeshPair* pairs;
+    int* zi;
+    int* wi;
+    double* wd;
+    int* counts;  // [pairs] merged contacts
+    double *pos, *nrm, *dep, *frame, *arm;  // [rows]
+};
+// The scratch of one pair (side 0 = a's part first, side 1 = b's behind it).
+struct PairView {
+    const MeshPair& P;
+    int nf0, nv0, nv;
+    int *count, *flag, *seed, *inside, *cand, *list, *order;
+    double *box, *world, *vpos, *vnrm, *vdep;
+    __device__ PairView(const MeshScratch& S, int k) : P(S.pairs[k]) {
+        nf0 = P.m[0].nf;
+        nv0 = P.m[0].nv;
+        nv = nv0 + P.m[1].nv;
+        const int nf = nf0 + P.m[1].nf;
+        count = S.zi + P.i0;
+        flag = count + 8;
+        seed = flag + nf;
+        inside = seed + nv;
+        cand = S.wi + P.j0;
+        list = cand + nf;
+        order = list + nv;
+        box = S.wd + P.d0;
+        world = box + 12;
+        vpos = world + 3LL * nv;
+        vnrm = vpos + 3LL * nv;
+        vdep = vnrm + 3LL * nv;
+    }
+    __device__ __forceinline__ int tri0(int side) const { return side ? nf0 : 0; }
+    __device__ __forceinline__ int vert0(int side) const { return side ? nv0 : 0; }
+    __device__ __forceinline__ void triangle(int side, int f, d3* t) const {
+        const int* F = P.m[side].F + 3 * f;
+        for (int k = 0; k < 3; ++k) t[k] = ldv(world, vert0(side) + F[k]);
+    }
+};
+__device__ __forceinline__ void tri_box(const d3* t, double* lo, double* hi) {
+    lo[0] = fmin(fmin(t[0].x, t[1].x), t[2].x); hi[0] = fmax(fmax(t[0].x, t[1].x), t[2].x);
+    lo[1] = fmin(fmin(t[0].y, t[1].y), t[2].y); hi[1] = fmax(fmax(t[0].y, t[1].y), t[2].y);
+    lo[2] = fmin(fmin(t[0].z, t[1].z), t[2].z); hi[2] = fmax(fmax(t[0].z, t[1].z), t[2].z);
+}
+
+// World vertices of one mesh of a pair and their box, one block (x: side, y: pair).
+__global__ void __launch_bounds__(512) mesh_world_kernel(const MeshScratch S) {
+    __shared__ double red[6][16];
+    const PairView V(S, blockIdx.y);
+    const int side = blockIdx.x;
+    const MeshDev& M = V.P.m[side];
+    double b[6] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY};  // lo, -hi
+    for (int v = threadIdx.x; v < M.nv; v += blockDim.x) {
+        const d3 w = world_vertex(M, v);
+        st3(V.world + 3LL * (V.vert0(side) + v), w);
+        b[0] = fmin(b[0], w.x); b[1] = fmin(b[1], w.y); b[2] = fmin(b[2], w.z);
+        b[3] = fmin(b[3], -w.x); b[4] = fmin(b[4], -w.y); b[5] = fmin(b[5], -w.z);
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        for (int o = 16; o > 0; o >>= 1) b[k] = fmin(b[k], __shfl_xor_sync(0xffffffffu, b[k], o));
+        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = b[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        double x = INFINITY;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) x = fmin(x, red[threadIdx.x][w]);
+        V.box[6 * side + threadIdx.x] = threadIdx.x < 3 ? x : -x;
+    }
+}
+
+// Triangles of either mesh whose box meets the other mesh's box: no other can
+// overlap one of the other mesh's triangles.  (y: pair)
+__global__ void __launch_bounds__(256) mesh_cull_kernel(const MeshScratch S) {
+    const PairView V(S, blockIdx.y);
+    for (int side = 0; side < 2; ++side) {
+        const double* o = V.box + 6 * (1 - side);
+        for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < V.P.m[side].nf; f += gridDim.x * blockDim.x) {
+            d3 t[3];
+            double lo[3], hi[3];
+            V.triangle(side, f, t);
+            tri_box(t, lo, hi);
+            if (hi[0] < o[0] || o[3] < lo[0] || hi[1] < o[1] || o[4] < lo[1] || hi[2] < o[2] || o[5] < lo[2]) continue;
+            V.cand[V.tri0(side) + atomicAdd(&V.count[side], 1)] = f;
         }
     }
 }
 
-// The vertices of flagged triangles (the seeds).
-__global__ void mesh_seed_kernel(const MeshDev M, const int* flag, int* seed) {
-    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < M.nf; f += gridDim.x * blockDim.x)
-        if (flag[f])
-            for (int k = 0; k < 3; ++k) seed[M.F[3 * f + k]] = 1;
+// Candidate triangle pairs whose boxes overlap and that no axis separates: both
+// triangles flagged, and their vertices listed as seeds (once each).  (y: pair)
+__global__ void __launch_bounds__(256) mesh_pairs_kernel(const MeshScratch S) {
+    const PairView V(S, blockIdx.y);
+    const int ca = V.count[0], cb = V.count[1];
+    const long long total = (long long)ca * cb;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
+         q += (long long)gridDim.x * blockDim.x) {
+        const int f[2] = {V.cand[q / cb], V.cand[V.nf0 + q % cb]};
+        d3 P[3], Q[3];
+        V.triangle(0, f[0], P);
+        V.triangle(1, f[1], Q);
+        double pl[3], ph[3], ql[3], qh[3];
+        tri_box(P, pl, ph);
+        tri_box(Q, ql, qh);
+        if (ph[0] < ql[0] || qh[0] < pl[0] || ph[1] < ql[1] || qh[1] < pl[1] || ph[2] < ql[2] || qh[2] < pl[2])
+            continue;
+        if (tri_separated(P, Q)) continue;
+        for (int side = 0; side < 2; ++side) {
+            if (atomicExch(&V.flag[V.tri0(side) + f[side]], 1)) continue;
+            for (int k = 0; k < 3; ++k) {
+                const int v = V.P.m[side].F[3 * f[side] + k];
+                if (!atomicExch(&V.seed[V.vert0(side) + v], 1))
+                    V.list[V.vert0(side) + atomicAdd(&V.count[2 + side], 1)] = v;
+            }
+        }
+    }
 }
 
-// Signed distance of every seed vertex of Q to mesh M, a warp per vertex (the
-// lanes split M's triangles; the closest is the first of least squared
+// Signed distance of every seed vertex to the other mesh M, a warp per vertex
+// (the lanes split M's triangles; the closest is the first of least squared
 // distance).  Inside vertices get their world position, depth and contact
-// normal (M's interpolated vertex normal times `sign`, so that it points from
-// the lower body to the higher).
-__global__ void __launch_bounds__(256) mesh_sdf_kernel(const MeshDev Q, const MeshDev M, const int* seed,
-                                                       double sign, int* inside, double* pos, double* nrm,
-                                                       double* depth) {
+// normal (M's interpolated vertex normal, from the lower body to the higher:
+// minus b's outward normal for a's vertices).  (y: pair)
+__global__ void __launch_bounds__(256) mesh_sdf_kernel(const MeshScratch S) {
+    const PairView V(S, blockIdx.y);
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < Q.nv; v += warps) {
-        if (!seed[v]) {
-            if (lane == 0) inside[v] = 0;
-            continue;
-        }
-        const d3 w = world_vertex(Q, v);
+    const int na = V.count[2], n = na + V.count[3];
+    for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < n; q += warps) {
+        const int side = q < na ? 0 : 1;
+        const int v = V.vert0(side) + V.list[V.vert0(side) + q - (side ? na : 0)];
+        const MeshDev& M = V.P.m[1 - side];
+        const double sign = side ? 1.0 : -1.0;
+        const d3 w = ldv(V.world, v);
         const d3 p = rot_t(M.R, sub3(w, M.c));
         double best = INFINITY;
         int bf = 0x7fffffff;
@@ -203,62 +297,123 @@ __global__ void __launch_bounds__(256) mesh_sdf_kernel(const MeshDev Q, const Me
                 bf = of;
             }
         }
-        if (lane == 0) {
-            int in = 0;
-            if (bf < M.nf) {
-                double b[3];
-                const int* tri = M.F + 3 * bf;
-                const d3 c = closest_on_triangle(p, ldv(M.V, tri[0]), ldv(M.V, tri[1]), ldv(M.V, tri[2]), b);
-                const int nsmall = (b[0] <= kPseudoEps) + (b[1] <= kPseudoEps) + (b[2] <= kPseudoEps);
-                d3 pn;
-                if (nsmall == 2) {  // a vertex: the corner whose coordinate is not small
-                    const int k = b[0] > kPseudoEps ? 0 : (b[1] > kPseudoEps ? 1 : 2);
-                    pn = ldv(M.vn, tri[k]);
-                } else if (nsmall == 1) {  // an edge: the one opposite the small coordinate
-                    const int k = b[0] <= kPseudoEps ? 0 : (b[1] <= kPseudoEps ? 1 : 2);
-                    pn = ldv(M.en, M.emap[3 * bf + k]);
-                } else {
-                    pn = ldv(M.fn, bf);
-                }
-                const double dist = (dot3(sub3(p, c), pn) >= 0 ? 1.0 : -1.0) * sqrt(best);
-                if (dist < 0) {
-                    in = 1;
-                    const d3 n = add3(add3(scl3(b[0], ldv(M.vn, tri[0])), scl3(b[1], ldv(M.vn, tri[1]))),
-                                      scl3(b[2], ldv(M.vn, tri[2])));
-                    const double nn = sqrt(dot3(n, n));
-                    const d3 nu = nn > 0 ? d3{n.x / nn, n.y / nn, n.z / nn} : n;
-                    const d3 nw = scl3(sign, rot(M.R, nu));
-                    pos[3 * v] = w.x; pos[3 * v + 1] = w.y; pos[3 * v + 2] = w.z;
-                    nrm[3 * v] = nw.x; nrm[3 * v + 1] = nw.y; nrm[3 * v + 2] = nw.z;
-                    depth[v] = -dist;
-                }
+        if (lane == 0 && bf < M.nf) {
+            double b[3];
+            const int* tri = M.F + 3 * bf;
+            const d3 c = closest_on_triangle(p, ldv(M.V, tri[0]), ldv(M.V, tri[1]), ldv(M.V, tri[2]), b);
+            const int nsmall = (b[0] <= kPseudoEps) + (b[1] <= kPseudoEps) + (b[2] <= kPseudoEps);
+            d3 pn;
+            if (nsmall == 2) {  // a vertex: the corner whose coordinate is not small
+                const int k = b[0] > kPseudoEps ? 0 : (b[1] > kPseudoEps ? 1 : 2);
+                pn = ldv(M.vn, tri[k]);
+            } else if (nsmall == 1) {  // an edge: the one opposite the small coordinate
+                const int k = b[0] <= kPseudoEps ? 0 : (b[1] <= kPseudoEps ? 1 : 2);
+                pn = ldv(M.en, M.emap[3 * bf + k]);
+            } else {
+                pn = ldv(M.fn, bf);
             }
-            inside[v] = in;
+            const double dist = (dot3(sub3(p, c), pn) >= 0 ? 1.0 : -1.0) * sqrt(best);
+            if (dist < 0) {
+                const d3 n3 = add3(add3(scl3(b[0], ldv(M.vn, tri[0])), scl3(b[1], ldv(M.vn, tri[1]))),
+                                   scl3(b[2], ldv(M.vn, tri[2])));
+                const double nn = sqrt(dot3(n3, n3));
+                const d3 nu = nn > 0 ? d3{n3.x / nn, n3.y / nn, n3.z / nn} : n3;
+                st3(V.vpos + 3LL * v, w);
+                st3(V.vnrm + 3LL * v, scl3(sign, rot(M.R, nu)));
+                V.vdep[v] = -dist;
+                V.inside[v] = 1;
+            }
         }
     }
 }
 
-// One thread: the inside vertices (A's in index order, then B's), sorted and
-// merged as every pair's points are, then frames and lever arms.
-__global__ void mesh_merge_kernel(int nva, int nvb, const int* inside, const double* pos, const double* nrm,
-                                  const double* depth, CPoint* pts, d3 ca, d3 cb, int cap, double* o_pos,
-                                  double* o_nrm, double* o_depth, double* o_frame, double* o_arm, int* n_out) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    int m = 0;
-    for (int v = 0; v < nva + nvb; ++v)
-        if (inside[v]) pts[m++] = CPoint{ldv(pos, v), ldv(nrm, v), depth[v]};
-    m = merge_points(pts, m);
-    for (int k = 0; k < m && k < cap; ++k) {
-        const CPoint& t = pts[k];
-        o_pos[3 * k] = t.p.x; o_pos[3 * k + 1] = t.p.y; o_pos[3 * k + 2] = t.p.z;
-        o_nrm[3 * k] = t.n.x; o_nrm[3 * k + 1] = t.n.y; o_nrm[3 * k + 2] = t.n.z;
-        o_depth[k] = fabs(t.depth);
-        frame_from_normal(t.n, o_frame + 9 * k);
-        const d3 a0 = sub3(t.p, ca), a1 = sub3(t.p, cb);
-        o_arm[6 * k] = a0.x; o_arm[6 * k + 1] = a0.y; o_arm[6 * k + 2] = a0.z;
-        o_arm[6 * k + 3] = a1.x; o_arm[6 * k + 4] = a1.y; o_arm[6 * k + 5] = a1.z;
+// Block-wide exclusive scan of one value per thread (256 threads); returns the total.
+__device__ __forceinline__ int block_scan256(int x, int* excl) {
+    __shared__ int part[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int s = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += y;
     }
-    *n_out = m;
+    if (lane == 31) part[warp] = s;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int w = 0; w < 8; ++w) {
+        before += w < warp ? part[w] : 0;
+        total += part[w];
+    }
+    __syncthreads();
+    *excl = before + s - x;
+    return total;
+}
+
+// One block per pair: the inside vertices (a's in index order, then b's) in the
+// order of merge_points (ranks on the position grid, ties in that order), runs of
+// near points merged by one thread each, then frames and lever arms.  One
+// thread walking all vertices and sorting took most of a query.
+__global__ void __launch_bounds__(256) mesh_merge_kernel(const MeshScratch S) {
+    const PairView V(S, blockIdx.x);
+    const int tid = threadIdx.x;
+    int m = 0, e;
+    for (int base = 0; base < V.nv; base += 256) {  // indices of the inside vertices, into the seeds' list
+        const int v = base + tid, in = v < V.nv ? V.inside[v] : 0;
+        const int t = block_scan256(in, &e);
+        if (in) V.list[m + e] = v;
+        m += t;
+    }
+    __syncthreads();
+    for (int i = tid; i < m; i += 256) {
+        const d3 p = ldv(V.vpos, V.list[i]);
+        const double x = grid_key(p.x), y = grid_key(p.y), z = grid_key(p.z);
+        int rank = 0;
+        for (int j = 0; j < m; ++j) {
+            const d3 o = ldv(V.vpos, V.list[j]);
+            const double ox = grid_key(o.x), oy = grid_key(o.y), oz = grid_key(o.z);
+            const bool less = ox != x ? ox < x : (oy != y ? oy < y : oz < z);
+            const bool tie = ox == x && oy == y && oz == z;
+            rank += less || (tie && j < i);
+        }
+        V.order[rank] = V.list[i];
+    }
+    __syncthreads();
+    const d3 ca = V.P.m[0].c, cb = V.P.m[1].c;
+    int done = 0;
+    for (int base = 0; base < m; base += 256) {
+        const int i = base + tid;
+        auto starts = [&](int k) {  // point k begins a run of near points
+            if (k == 0) return true;
+            const d3 d = sub3(ldv(V.vpos, V.order[k]), ldv(V.vpos, V.order[k - 1]));
+            return dot3(d, d) > 1e-8;
+        };
+        const bool first = i < m && starts(i);
+        const int t = block_scan256(first ? 1 : 0, &e);
+        if (first) {
+            const int v = V.order[i];
+            d3 nrm = ldv(V.vnrm, v);
+            double depth = V.vdep[v];
+            int j = i + 1;
+            for (; j < m && !starts(j); ++j) {
+                nrm = add3(nrm, ldv(V.vnrm, V.order[j]));
+                depth = fmin(V.vdep[V.order[j]], depth);
+            }
+            if (j - i > 1) {
+                const double nn = sqrt(dot3(nrm, nrm));
+                nrm = (nn > 0) ? scl3(1.0 / nn, nrm) : nrm;
+            }
+            const long long r = V.P.row0 + done + e;
+            const d3 p = ldv(V.vpos, v);
+            st3(S.pos + 3 * r, p);
+            st3(S.nrm + 3 * r, nrm);
+            S.dep[r] = fabs(depth);
+            frame_from_normal(nrm, S.frame + 9 * r);
+            st3(S.arm + 6 * r, sub3(p, ca));
+            st3(S.arm + 6 * r + 3, sub3(p, cb));
+        }
+        done += t;
+    }
+    if (tid == 0) S.counts[blockIdx.x] = done;
 }
 
 // Pair k's merged contacts (rows of its own region, region k starting at row
@@ -429,15 +584,13 @@ extern "C" int pdc_mesh_create(int32_t n_verts, const double* verts, int32_t n_t
     return PDC_OK;
 }
 
-extern "C" int pdc_mesh_contacts(const pdc_mesh* a, const double pose_a[7], const pdc_mesh* b,
-                                 const double pose_b[7], int32_t max_points, double* pos, double* normal,
-                                 double* depth, double* frame, double* arm, int32_t* n_points) {
+// Contacts of n_pairs pairs (arguments checked): one set of launches for all of
+// them, one device allocation, packed rows into the host arrays.
+static int mesh_query(int32_t n_pairs, const pdc_mesh* const* a, const double* poses_a, const pdc_mesh* const* b,
+                      const double* poses_b, int32_t max_points, double* pos, double* normal, double* depth,
+                      double* frame, double* arm, int32_t* counts, long long* total_out, const char* who) {
     pdc_solver* s = nullptr;
-    if (!a || !b || !pose_a || !pose_b || !n_points || max_points < 0 ||
-        (max_points > 0 && (!pos || !normal || !depth || !frame || !arm)))
-        return fail(s, PDC_EINVAL, "pdc_mesh_contacts: null argument");
-    if (a->device != b->device) return fail(s, PDC_EINVAL, "pdc_mesh_contacts: meshes on different devices");
-    CK(cudaSetDevice(a->device), "cudaSetDevice");
+    CK(cudaSetDevice(a[0]->device), "cudaSetDevice");
     auto dev = [](const pdc_mesh* m, const double* pose) {
         pdc::MeshDev d;
         d.nv = m->nv; d.nf = m->nf;
@@ -446,59 +599,102 @@ extern "C" int pdc_mesh_contacts(const pdc_mesh* a, const double pose_a[7], cons
         d.c = pdc::d3{pose[0], pose[1], pose[2]};
         return d;
     };
-    const pdc::MeshDev A = dev(a, pose_a), B = dev(b, pose_b);
-    const int nv = a->nv + b->nv;
+    std::vector<pdc::MeshPair> pairs(n_pairs);
+    std::vector<long long> row0(n_pairs);
+    long long ni = 0, nj = 0, nd = 0, nrows = 0, most_tris = 0;
+    for (int k = 0; k < n_pairs; ++k) {
+        const long long nv = (long long)a[k]->nv + b[k]->nv, nf = (long long)a[k]->nf + b[k]->nf;
+        pdc::MeshPair& P = pairs[k];
+        P.m[0] = dev(a[k], poses_a + 7LL * k);
+        P.m[1] = dev(b[k], poses_b + 7LL * k);
+        P.i0 = ni; ni += 8 + nf + 2 * nv;
+        P.j0 = nj; nj += nf + 2 * nv;
+        P.d0 = nd; nd += 12 + 10 * nv;
+        P.row0 = row0[k] = nrows; nrows += nv;  // a pair merges at most its inside vertices
+        most_tris = std::max(most_tris, nf);
+    }
+    const long long cap = std::max<long long>(1, std::min<long long>(max_points, nrows));
+    Arena A;
+    pdc::MeshScratch S;
+    pdc::MeshPair* d_pairs = nullptr;
+    long long* d_row0 = nullptr;
+    double* out = nullptr;
+    auto carve_query = [&](Arena& q) {
+        q.reset();
+        d_pairs = q.take<pdc::MeshPair>(n_pairs);
+        d_row0 = q.take<long long>(n_pairs);
+        S.pairs = d_pairs;
+        S.zi = q.take<int>(ni);
+        S.wi = q.take<int>(nj);
+        S.wd = q.take<double>(nd);
+        S.counts = q.take<int>(n_pairs);
+        S.pos = q.take<double>(22 * nrows);
+        S.nrm = S.pos + 3 * nrows;
+        S.dep = S.nrm + 3 * nrows;
+        S.frame = S.dep + nrows;
+        S.arm = S.frame + 9 * nrows;
+        out = q.take<double>(22 * cap);
+        return q.off + 256;
+    };
+    const size_t need = carve_query(A);
     DevScratch sc;
-    int *flag_a, *flag_b, *seed, *inside, *n_out;
-    double *vpos, *vnrm, *vdep, *o_pos, *o_nrm, *o_dep, *o_frame, *o_arm;
-    pdc::CPoint* pts;
-    const int cap = std::max(1, std::min(max_points, nv));
-    cudaError_t e = sc.get(&flag_a, a->nf);
-    if (e == cudaSuccess) e = sc.get(&flag_b, b->nf);
-    if (e == cudaSuccess) e = sc.get(&seed, nv);
-    if (e == cudaSuccess) e = sc.get(&inside, nv);
-    if (e == cudaSuccess) e = sc.get(&n_out, 1);
-    if (e == cudaSuccess) e = sc.get(&vpos, 3LL * nv);
-    if (e == cudaSuccess) e = sc.get(&vnrm, 3LL * nv);
-    if (e == cudaSuccess) e = sc.get(&vdep, nv);
-    if (e == cudaSuccess) e = sc.get(&pts, nv);
-    if (e == cudaSuccess) e = sc.get(&o_pos, 3LL * cap);
-    if (e == cudaSuccess) e = sc.get(&o_nrm, 3LL * cap);
-    if (e == cudaSuccess) e = sc.get(&o_dep, cap);
-    if (e == cudaSuccess) e = sc.get(&o_frame, 9LL * cap);
-    if (e == cudaSuccess) e = sc.get(&o_arm, 6LL * cap);
-    if (e != cudaSuccess) return cuda_fail(s, e, "pdc_mesh_contacts: scratch");
-    CK(cudaMemset(flag_a, 0, sizeof(int) * a->nf), "memset");
-    CK(cudaMemset(flag_b, 0, sizeof(int) * b->nf), "memset");
-    CK(cudaMemset(seed, 0, sizeof(int) * nv), "memset");
+    char* mem = nullptr;
+    const cudaError_t e = sc.get(&mem, need);
+    if (e != cudaSuccess) return cuda_fail(s, e, who);
+    A.base = mem;
+    carve_query(A);
+    CK(cudaMemcpyAsync(d_pairs, pairs.data(), sizeof(pdc::MeshPair) * n_pairs, cudaMemcpyHostToDevice), "H2D pairs");
+    CK(cudaMemcpyAsync(d_row0, row0.data(), sizeof(long long) * n_pairs, cudaMemcpyHostToDevice), "H2D rows");
+    CK(cudaMemsetAsync(S.zi, 0, sizeof(int) * ni), "memset");
     int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a->device);
-    const long long pairs = (long long)a->nf * b->nf;
-    const int pblocks = (int)std::max(1LL, std::min<long long>((pairs + 255) / 256, 16LL * sms));
-    pdc::mesh_pairs_kernel<<<pblocks, 256>>>(A, B, flag_a, flag_b);
-    pdc::mesh_seed_kernel<<<std::max(1, std::min((a->nf + 255) / 256, 8 * sms)), 256>>>(A, flag_a, seed);
-    pdc::mesh_seed_kernel<<<std::max(1, std::min((b->nf + 255) / 256, 8 * sms)), 256>>>(B, flag_b, seed + a->nv);
-    const int wblocks_a = std::max(1, std::min((a->nv + 7) / 8, 16 * sms));
-    const int wblocks_b = std::max(1, std::min((b->nv + 7) / 8, 16 * sms));
-    // a's vertices in b (normal from a to b: minus b's outward normal), then b's in a
-    pdc::mesh_sdf_kernel<<<wblocks_a, 256>>>(A, B, seed, -1.0, inside, vpos, vnrm, vdep);
-    pdc::mesh_sdf_kernel<<<wblocks_b, 256>>>(B, A, seed + a->nv, 1.0, inside + a->nv, vpos + 3LL * a->nv,
-                                             vnrm + 3LL * a->nv, vdep + a->nv);
-    pdc::mesh_merge_kernel<<<1, 1>>>(a->nv, b->nv, inside, vpos, vnrm, vdep, pts, A.c, B.c, cap, o_pos, o_nrm,
-                                     o_dep, o_frame, o_arm, n_out);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a[0]->device);
+    for (int k0 = 0; k0 < n_pairs; k0 += 32768) {  // grid.y
+        const int n = std::min(n_pairs - k0, 32768);
+        pdc::MeshScratch Q = S;
+        Q.pairs += k0;
+        Q.counts += k0;
+        // blocks per pair: enough to fill the GPU, no more than the largest pair's triangles need
+        const int fill = std::max(1, (16 * sms + n - 1) / n);
+        const int gf = (int)std::max(1LL, std::min<long long>((most_tris + 255) / 256, fill));
+        pdc::mesh_world_kernel<<<dim3(2, n), 512>>>(Q);
+        pdc::mesh_cull_kernel<<<dim3(gf, n), 256>>>(Q);
+        pdc::mesh_pairs_kernel<<<dim3(fill, n), 256>>>(Q);
+        pdc::mesh_sdf_kernel<<<dim3(fill, n), 256>>>(Q);
+        pdc::mesh_merge_kernel<<<n, 256>>>(Q);
+    }
+    double *o_nrm = out + 3 * cap, *o_dep = o_nrm + 3 * cap, *o_frame = o_dep + cap, *o_arm = o_frame + 9 * cap;
+    pdc::mesh_gather_kernel<<<n_pairs, 128>>>(n_pairs, S.counts, d_row0, S.pos, S.nrm, S.dep, S.frame, S.arm,
+                                              (int)cap, out, o_nrm, o_dep, o_frame, o_arm);
     CK(cudaGetLastError(), "launch mesh kernels");
-    int m = 0;
-    CK(cudaMemcpy(&m, n_out, sizeof(int), cudaMemcpyDeviceToHost), "D2H count");
-    const int w = std::min(m, max_points);
+    CK(cudaMemcpy(counts, S.counts, sizeof(int32_t) * n_pairs, cudaMemcpyDeviceToHost), "D2H counts");
+    long long total = 0;
+    for (int k = 0; k < n_pairs; ++k) total += counts[k];
+    const long long w = std::min<long long>(total, max_points);
     if (w > 0) {
-        CK(cudaMemcpy(pos, o_pos, 3 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
-        CK(cudaMemcpy(normal, o_nrm, 3 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
-        CK(cudaMemcpy(depth, o_dep, sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
-        CK(cudaMemcpy(frame, o_frame, 9 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
+        CK(cudaMemcpyAsync(pos, out, 3 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
+        CK(cudaMemcpyAsync(normal, o_nrm, 3 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
+        CK(cudaMemcpyAsync(depth, o_dep, sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
+        CK(cudaMemcpyAsync(frame, o_frame, 9 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
         CK(cudaMemcpy(arm, o_arm, 6 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
     }
-    *n_points = m;
+    *total_out = total;
     return PDC_OK;
+}
+
+extern "C" int pdc_mesh_contacts(const pdc_mesh* a, const double pose_a[7], const pdc_mesh* b,
+                                 const double pose_b[7], int32_t max_points, double* pos, double* normal,
+                                 double* depth, double* frame, double* arm, int32_t* n_points) {
+    pdc_solver* s = nullptr;
+    if (!a || !b || !pose_a || !pose_b || !n_points || max_points < 0 ||
+        (max_points > 0 && (!pos || !normal || !depth || !frame || !arm)))
+        return fail(s, PDC_EINVAL, "pdc_mesh_contacts: null argument");
+    if (a->device != b->device) return fail(s, PDC_EINVAL, "pdc_mesh_contacts: meshes on different devices");
+    int32_t count = 0;
+    long long total = 0;
+    const int rc = mesh_query(1, &a, pose_a, &b, pose_b, max_points, pos, normal, depth, frame, arm, &count, &total,
+                              "pdc_mesh_contacts: scratch");
+    if (rc == PDC_OK) *n_points = count;
+    return rc;
 }
 
 extern "C" int pdc_mesh_contacts_pairs(int32_t n_pairs, const pdc_mesh* const* a, const double* poses_a,
@@ -517,92 +713,9 @@ extern "C" int pdc_mesh_contacts_pairs(int32_t n_pairs, const pdc_mesh* const* a
         if (a[k]->device != a[0]->device || b[k]->device != a[0]->device)
             return fail(s, PDC_EINVAL, "pdc_mesh_contacts_pairs: meshes on different devices");
     }
-    CK(cudaSetDevice(a[0]->device), "cudaSetDevice");
-    // per-pair regions: ints (flags of a's and b's triangles, seeds and inside
-    // flags of both meshes' vertices), doubles (inside positions, normals and
-    // depths, then the merged rows), points (the merge's work array)
-    std::vector<long long> i0(n_pairs), d0(n_pairs), p0(n_pairs), row0(n_pairs);
-    long long ni = 0, nd = 0, np = 0, nrows = 0;
-    for (int k = 0; k < n_pairs; ++k) {
-        const long long nv = (long long)a[k]->nv + b[k]->nv;
-        i0[k] = ni; ni += (long long)a[k]->nf + b[k]->nf + 2 * nv;
-        d0[k] = nd; nd += 7 * nv;
-        p0[k] = np; np += nv;
-        row0[k] = nrows; nrows += nv;  // a pair merges at most its inside vertices
-    }
-    const long long cap = std::max<long long>(1, std::min<long long>(max_points, nrows));
-    DevScratch sc;
-    int *ibuf, *d_counts;
-    double *dbuf, *rows, *o_pos, *o_nrm, *o_dep, *o_frame, *o_arm;
-    long long* d_row0;
-    pdc::CPoint* pts;
-    cudaError_t e = sc.get(&ibuf, ni);
-    if (e == cudaSuccess) e = sc.get(&d_counts, n_pairs);
-    if (e == cudaSuccess) e = sc.get(&d_row0, n_pairs);
-    if (e == cudaSuccess) e = sc.get(&dbuf, nd);
-    if (e == cudaSuccess) e = sc.get(&rows, 22 * nrows);
-    if (e == cudaSuccess) e = sc.get(&pts, np);
-    if (e == cudaSuccess) e = sc.get(&o_pos, 22 * cap);
-    if (e != cudaSuccess) return cuda_fail(s, e, "pdc_mesh_contacts_pairs: scratch");
-    o_nrm = o_pos + 3 * cap; o_dep = o_nrm + 3 * cap; o_frame = o_dep + cap; o_arm = o_frame + 9 * cap;
-    double* r_pos = rows;
-    double* r_nrm = r_pos + 3 * nrows;
-    double* r_dep = r_nrm + 3 * nrows;
-    double* r_frame = r_dep + nrows;
-    double* r_arm = r_frame + 9 * nrows;
-    CK(cudaMemset(ibuf, 0, sizeof(int) * ni), "memset");
-    CK(cudaMemcpy(d_row0, row0.data(), sizeof(long long) * n_pairs, cudaMemcpyHostToDevice), "H2D rows");
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a[0]->device);
-    auto dev = [](const pdc_mesh* m, const double* pose) {
-        pdc::MeshDev d;
-        d.nv = m->nv; d.nf = m->nf;
-        d.V = m->V; d.F = m->F; d.fn = m->fn; d.vn = m->vn; d.en = m->en; d.emap = m->emap;
-        host_quat_to_R(pose + 3, d.R);
-        d.c = pdc::d3{pose[0], pose[1], pose[2]};
-        return d;
-    };
-    for (int k = 0; k < n_pairs; ++k) {  // the kernels of pdc_mesh_contacts, pair after pair on one stream
-        const pdc_mesh *ma = a[k], *mb = b[k];
-        const pdc::MeshDev A = dev(ma, poses_a + 7LL * k), B = dev(mb, poses_b + 7LL * k);
-        const int nv = ma->nv + mb->nv;
-        int* flag_a = ibuf + i0[k];
-        int* flag_b = flag_a + ma->nf;
-        int* seed = flag_b + mb->nf;
-        int* inside = seed + nv;
-        double* vpos = dbuf + d0[k];
-        double* vnrm = vpos + 3LL * nv;
-        double* vdep = vnrm + 3LL * nv;
-        const long long r = row0[k];
-        const long long pairs = (long long)ma->nf * mb->nf;
-        const int pblocks = (int)std::max(1LL, std::min<long long>((pairs + 255) / 256, 16LL * sms));
-        pdc::mesh_pairs_kernel<<<pblocks, 256>>>(A, B, flag_a, flag_b);
-        pdc::mesh_seed_kernel<<<std::max(1, std::min((ma->nf + 255) / 256, 8 * sms)), 256>>>(A, flag_a, seed);
-        pdc::mesh_seed_kernel<<<std::max(1, std::min((mb->nf + 255) / 256, 8 * sms)), 256>>>(B, flag_b,
-                                                                                           seed + ma->nv);
-        const int wblocks_a = std::max(1, std::min((ma->nv + 7) / 8, 16 * sms));
-        const int wblocks_b = std::max(1, std::min((mb->nv + 7) / 8, 16 * sms));
-        pdc::mesh_sdf_kernel<<<wblocks_a, 256>>>(A, B, seed, -1.0, inside, vpos, vnrm, vdep);
-        pdc::mesh_sdf_kernel<<<wblocks_b, 256>>>(B, A, seed + ma->nv, 1.0, inside + ma->nv, vpos + 3LL * ma->nv,
-                                                 vnrm + 3LL * ma->nv, vdep + ma->nv);
-        pdc::mesh_merge_kernel<<<1, 1>>>(ma->nv, mb->nv, inside, vpos, vnrm, vdep, pts + p0[k], A.c, B.c, nv,
-                                         r_pos + 3 * r, r_nrm + 3 * r, r_dep + r, r_frame + 9 * r, r_arm + 6 * r,
-                                         d_counts + k);
-    }
-    pdc::mesh_gather_kernel<<<n_pairs, 128>>>(n_pairs, d_counts, d_row0, r_pos, r_nrm, r_dep, r_frame, r_arm,
-                                              (int)cap, o_pos, o_nrm, o_dep, o_frame, o_arm);
-    CK(cudaGetLastError(), "launch mesh kernels");
-    CK(cudaMemcpy(counts, d_counts, sizeof(int32_t) * n_pairs, cudaMemcpyDeviceToHost), "D2H counts");
     long long total = 0;
-    for (int k = 0; k < n_pairs; ++k) total += counts[k];
-    const long long w = std::min<long long>(total, max_points);
-    if (w > 0) {
-        CK(cudaMemcpy(pos, o_pos, 3 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
-        CK(cudaMemcpy(normal, o_nrm, 3 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
-        CK(cudaMemcpy(depth, o_dep, sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
-        CK(cudaMemcpy(frame, o_frame, 9 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
-        CK(cudaMemcpy(arm, o_arm, 6 * sizeof(double) * w, cudaMemcpyDeviceToHost), "D2H contacts");
-    }
-    *n_points = (int32_t)std::min<long long>(total, 0x7fffffffLL);
-    return PDC_OK;
+    const int rc = mesh_query(n_pairs, a, poses_a, b, poses_b, max_points, pos, normal, depth, frame, arm, counts,
+                              &total, "pdc_mesh_contacts_pairs: scratch");
+    if (rc == PDC_OK) *n_points = (int32_t)std::min<long long>(total, 0x7fffffffLL);
+    return rc;
 }
