@@ -365,19 +365,10 @@ __device__ __forceinline__ BodyG load_body(const WorldPtrs& W, int gb) {
     g.stat = W.is_static[gb] != 0;
     return g;
 }
-__device__ __forceinline__ bool aabb_overlap(const BodyG& a, const BodyG& b) {
-    if (a.type == SHAPE_PLANE || b.type == SHAPE_PLANE) return true;
-    double ea[3], eb[3];
-    for (int r = 0; r < 3; ++r) {
-        if (a.type == SHAPE_SPHERE) ea[r] = a.h[0];
-        else ea[r] = fabs(a.R[3 * r]) * a.h[0] + fabs(a.R[3 * r + 1]) * a.h[1] + fabs(a.R[3 * r + 2]) * a.h[2];
-        if (b.type == SHAPE_SPHERE) eb[r] = b.h[0];
-        else eb[r] = fabs(b.R[3 * r]) * b.h[0] + fabs(b.R[3 * r + 1]) * b.h[1] + fabs(b.R[3 * r + 2]) * b.h[2];
-    }
-    const double dc[3] = {b.c.x - a.c.x, b.c.y - a.c.y, b.c.z - a.c.z};
-    for (int r = 0; r < 3; ++r)
-        if (fabs(dc[r]) > ea[r] + eb[r]) return false;
-    return true;
+// half extent of a body's AABB along axis r (planes have none)
+__device__ __forceinline__ double body_extent(const BodyG& a, int r) {
+    if (a.type == SHAPE_SPHERE) return a.h[0];
+    return fabs(a.R[3 * r]) * a.h[0] + fabs(a.R[3 * r + 1]) * a.h[1] + fabs(a.R[3 * r + 2]) * a.h[2];
 }
 
 // All contact points of pair (a, b), a having the lower id; normal from a to b.

@@ -271,7 +271,7 @@ extern "C" int pdc_server_tick(pdc_server* v, void* stream) {
         CK(cudaStreamBeginCapture(v->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
         const int gb = std::max(1, (int)std::min<long long>((v->NB + 255) / 256, s->num_sms * 8));
         pdc::prepare_bodies_kernel<<<gb, 256, 0, v->stream>>>(v->W, v->body_scene, (int)v->NB);
-        pdc::collide_kernel<<<std::max(1, std::min(v->S, s->num_sms * 4)), 256, 0, v->stream>>>(v->W);
+        pdc::collide_kernel<<<std::max(1, std::min(v->S, s->num_sms * 32)), pdc::kCollideThreads, 0, v->stream>>>(v->W);
         int rc = launch(s, v->P, v->stream);
         pdc::integrate_kernel<<<gb, 256, 0, v->stream>>>(v->W, v->body_scene, (int)v->NB);
         cudaGraph_t g = nullptr;

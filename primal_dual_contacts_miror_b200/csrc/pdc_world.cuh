@@ -32,15 +32,43 @@ __global__ void prepare_bodies_kernel(const __grid_constant__ WorldPtrs W, const
     }
 }
 
-__device__ __forceinline__ long long pair_row_start(long long i, long long n) { return i * (2 * n - i - 1) / 2; }
+// Contact detection of one scene per block.  All pairs (i < j) in lexicographic
+// order go through the AABB test, kPairRounds x kCollideThreads at a time, and the
+// ones that pass enter a ring in that order; as soon as the ring holds a candidate
+// for every thread the narrow phase runs on them, and a scan of the point counts
+// gives the offsets, so the contact order is (i, j, position) exactly as the
+// reference sorts it.  The narrow phase (a separating-axis test with clipping in
+// local memory) is what the time goes to: it runs once per candidate, with all
+// lanes on candidates, where a contiguous range of pairs per thread left most lanes
+// idle and needed a second pass for the offsets.  128 threads, since the narrow
+// phase takes nearly all registers a thread can have: two blocks per SM, and small
+// scenes leave fewer lanes idle than with 256.
+constexpr int kCollideThreads = 128;
+constexpr int kPairRounds = 4;       // AABB tests per thread between two barriers
+constexpr int kCollideBodies = 512;  // bodies whose boxes are kept in shared memory
+constexpr int kCandidates = 1024;    // ring: a power of two >= (1 + kPairRounds) * kCollideThreads
+static_assert(kCandidates >= (1 + kPairRounds) * kCollideThreads, "candidate ring too small");
 
-// Contact detection of one scene per block: all pairs (i < j) in lexicographic
-// order split into contiguous per-thread chunks; a counting pass and a scan give
-// every thread its write offset, a second pass writes the merged points, so the
-// contact order is (i, j, position) exactly as the reference sorts it.
-__global__ void __launch_bounds__(256) collide_kernel(const __grid_constant__ WorldPtrs W) {
-    __shared__ int s_off[257];
-    const int tid = threadIdx.x, nt = blockDim.x;
+struct AabbG {
+    double c[3], e[3];
+    int flags;  // 1: static, 2: plane (meets everything)
+};
+__device__ __forceinline__ AabbG load_aabb(const WorldPtrs& W, int gb) {
+    const BodyG g = load_body(W, gb);
+    AabbG x;
+    x.c[0] = g.c.x; x.c[1] = g.c.y; x.c[2] = g.c.z;
+    for (int r = 0; r < 3; ++r) x.e[r] = body_extent(g, r);
+    x.flags = (g.stat ? 1 : 0) | (g.type == SHAPE_PLANE ? 2 : 0);
+    return x;
+}
+
+__global__ void __launch_bounds__(kCollideThreads) collide_kernel(const __grid_constant__ WorldPtrs W) {
+    constexpr int nw = kCollideThreads / 32;
+    __shared__ double s_box[6][kCollideBodies];
+    __shared__ unsigned char s_flag[kCollideBodies];
+    __shared__ int2 s_cand[kCandidates];
+    __shared__ int s_cnt[kPairRounds * nw], s_sum[nw];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int s = blockIdx.x; s < W.n_scenes; s += gridDim.x) {
         if (W.skip && W.skip[s]) continue;  // large scene: sort-based path
         if (W.dt[s] == 0.0) {  // scene done with its adaptive substeps: no contacts, no motion
@@ -52,73 +80,123 @@ __global__ void __launch_bounds__(256) collide_kernel(const __grid_constant__ Wo
         }
         const int b0 = W.body_off[s], nb = W.body_cnt ? W.body_cnt[s] : W.body_off[s + 1] - b0;
         const int cap0 = W.contact_cap[s], cap = W.cap_cnt ? W.cap_cnt[s] : W.contact_cap[s + 1] - cap0;
+        __syncthreads();  // the previous scene's boxes are no longer read
+        for (int b = tid; b < min(nb, kCollideBodies); b += kCollideThreads) {
+            const AabbG x = load_aabb(W, b0 + b);
+            for (int r = 0; r < 3; ++r) {
+                s_box[r][b] = x.c[r];
+                s_box[3 + r][b] = x.e[r];
+            }
+            s_flag[b] = (unsigned char)x.flags;
+        }
+        __syncthreads();
+        auto aabb = [&](int b) {
+            if (b >= kCollideBodies) return load_aabb(W, b0 + b);
+            AabbG x;
+            for (int r = 0; r < 3; ++r) {
+                x.c[r] = s_box[r][b];
+                x.e[r] = s_box[3 + r][b];
+            }
+            x.flags = s_flag[b];
+            return x;
+        };
+        // the pair `tid` of the scene in lexicographic order, then every kCollideThreads-th
+        int i = 0, j = 1 + tid;
+        auto normalise = [&]() {
+            while (i < nb - 1 && j >= nb) {
+                ++i;
+                j += i + 1 - nb;
+            }
+        };
+        normalise();
         const long long npairs = (long long)nb * (nb - 1) / 2;
-        const long long chunk = (npairs + nt - 1) / nt;
-        const long long p0 = tid * chunk, p1 = min(npairs, p0 + chunk);
-        for (int pass = 0; pass < 2; ++pass) {
-            int off = pass ? s_off[tid] : 0;
-            int cnt = 0;
-            if (p0 < p1) {
-                // first pair of the chunk
-                long long i = (long long)((2.0 * nb - 1 - sqrt((2.0 * nb - 1) * (2.0 * nb - 1) - 8.0 * p0)) * 0.5);
-                if (i < 0) i = 0;
-                while (i > 0 && pair_row_start(i, nb) > p0) --i;
-                while (i + 1 < nb && pair_row_start(i + 1, nb) <= p0) ++i;
-                long long j = i + 1 + (p0 - pair_row_start(i, nb));
-                for (long long p = p0; p < p1; ++p) {
-                    const int gi = b0 + (int)i, gj = b0 + (int)j;
-                    const bool si = W.is_static[gi] != 0, sj = W.is_static[gj] != 0;
-                    if (!(si && sj)) {
-                        const BodyG A = load_body(W, gi), Bg = load_body(W, gj);
-                        if (aabb_overlap(A, Bg)) {
-                            CPoint pts[PDC_MAX_PAIR_POINTS];
-                            int m = pair_points(A, Bg, pts);
-                            m = merge_points(pts, m);
-                            if (pass) {
-                                for (int q = 0; q < m; ++q, ++off) {
-                                    if (off >= cap) continue;
-                                    const long long gc = cap0 + off;
-                                    W.cbody[2 * gc] = (int)i;
-                                    W.cbody[2 * gc + 1] = (int)j;
-                                    frame_from_normal(pts[q].n, W.frame + 9 * gc);
-                                    st3(W.arm + 6 * gc, sub3(pts[q].p, A.c));
-                                    st3(W.arm + 6 * gc + 3, sub3(pts[q].p, Bg.c));
-                                    W.depth[gc] = fabs(pts[q].depth);
-                                    st3(W.cpos + 3 * gc, pts[q].p);
-                                }
-                            } else {
-                                cnt += m;
-                            }
+        int head = 0, tail = 0;  // candidates taken and entered
+        int off = 0;             // points written
+        for (long long done = 0; done < npairs || head < tail;) {
+            if (done < npairs) {
+                unsigned hit = 0, before[kPairRounds];
+                int pi[kPairRounds], pj[kPairRounds];
+#pragma unroll
+                for (int k = 0; k < kPairRounds; ++k) {
+                    bool f = false;
+                    pi[k] = i;
+                    pj[k] = j;
+                    if (i < nb - 1) {
+                        const AabbG A = aabb(i), B = aabb(j);
+                        if (!(A.flags & B.flags & 1)) {
+                            f = true;
+                            if (!((A.flags | B.flags) & 2))
+                                for (int r = 0; r < 3; ++r)
+                                    if (fabs(B.c[r] - A.c[r]) > A.e[r] + B.e[r]) f = false;
                         }
+                        j += kCollideThreads;
+                        normalise();
                     }
-                    if (++j == nb) {
-                        ++i;
-                        j = i + 1;
-                    }
+                    const unsigned m = __ballot_sync(0xffffffffu, f);
+                    if (f) hit |= 1u << k;
+                    before[k] = __popc(m & ((1u << lane) - 1u));
+                    if (lane == 0) s_cnt[k * nw + warp] = __popc(m);
                 }
+                __syncthreads();
+                int base = tail;
+#pragma unroll
+                for (int k = 0; k < kPairRounds; ++k)
+#pragma unroll
+                    for (int w = 0; w < nw; ++w) {
+                        if (w == warp && (hit >> k & 1u))
+                            s_cand[(base + before[k]) & (kCandidates - 1)] = make_int2(pi[k], pj[k]);
+                        base += s_cnt[k * nw + w];
+                    }
+                tail = base;
+                done += kPairRounds * kCollideThreads;
+                __syncthreads();
             }
-            if (!pass) {
-                s_off[tid] = cnt;
+            // narrow phase on full rounds, and on what is left once every pair is tested
+            while (tail - head >= kCollideThreads || (done >= npairs && head < tail)) {
+                int m = 0;
+                int2 c = make_int2(0, 0);
+                CPoint pts[PDC_MAX_PAIR_POINTS];
+                d3 ca, cb;
+                if (head + tid < tail) {
+                    c = s_cand[(head + tid) & (kCandidates - 1)];
+                    const BodyG A = load_body(W, b0 + c.x), Bg = load_body(W, b0 + c.y);
+                    ca = A.c;
+                    cb = Bg.c;
+                    m = pair_points(A, Bg, pts);
+                    m = merge_points(pts, m);
+                }
+                int pre = m;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, pre, o);
+                    if (lane >= o) pre += v;
+                }
+                if (lane == 31) s_sum[warp] = pre;
                 __syncthreads();
-                if (tid == 0) {
-                    int acc = 0;
-                    for (int t = 0; t < nt; ++t) {
-                        const int c = s_off[t];
-                        s_off[t] = acc;
-                        acc += c;
-                    }
-                    s_off[nt] = acc;
+                int at = off + pre - m;
+#pragma unroll
+                for (int w = 0; w < nw; ++w) {
+                    if (w < warp) at += s_sum[w];
+                    off += s_sum[w];
                 }
                 __syncthreads();
+                for (int q = 0; q < m; ++q, ++at) {
+                    if (at >= cap) continue;
+                    const long long gc = cap0 + at;
+                    W.cbody[2 * gc] = c.x;
+                    W.cbody[2 * gc + 1] = c.y;
+                    frame_from_normal(pts[q].n, W.frame + 9 * gc);
+                    st3(W.arm + 6 * gc, sub3(pts[q].p, ca));
+                    st3(W.arm + 6 * gc + 3, sub3(pts[q].p, cb));
+                    W.depth[gc] = fabs(pts[q].depth);
+                    st3(W.cpos + 3 * gc, pts[q].p);
+                }
+                head = min(tail, head + kCollideThreads);
             }
         }
-        __syncthreads();
         if (tid == 0) {
-            const int total = s_off[nt];
-            W.ccount[s] = min(total, cap);
-            W.overflow[s] = max(0, total - cap);
+            W.ccount[s] = min(off, cap);
+            W.overflow[s] = max(0, off - cap);
         }
-        __syncthreads();
     }
 }
 
@@ -286,8 +364,8 @@ static int world_collide(pdc_world* w, cudaStream_t st) {
     const int gb = std::max(1, std::min((w->nb + 255) / 256, s->num_sms * 8));
     pdc::prepare_bodies_kernel<<<gb, 256, 0, st>>>(w->W, w->body_scene, w->nb);
     CK(cudaGetLastError(), "launch prepare_bodies_kernel");
-    const int gc = std::max(1, std::min(w->ns, s->num_sms * 4));
-    pdc::collide_kernel<<<gc, 256, 0, st>>>(w->W);
+    const int gc = std::max(1, std::min(w->ns, s->num_sms * 32));  // more than fit at once: blocks balance the scenes
+    pdc::collide_kernel<<<gc, pdc::kCollideThreads, 0, st>>>(w->W);
     CK(cudaGetLastError(), "launch collide_kernel");
     pdc::LargeCollide& L = w->L;
     const int gl = s->num_sms * 8;
@@ -298,9 +376,10 @@ static int world_collide(pdc_world* w, cudaStream_t st) {
         size_t tb = L.temp_bytes;
         CK(cub::DeviceRadixSort::SortPairs(L.temp, tb, L.key, L.key_s, L.val, L.val_s, L.nb_max, 0, 32, st),
            "sort bodies");
-        pdc::large_sweep_kernel<<<gl, 256, 0, st>>>(w->W, L, sc);
+        const dim3 gs(std::min((L.nb_max + pdc::kSweepTile - 1) / pdc::kSweepTile, 1 << 16), pdc::kSweepSplit);
+        pdc::large_sweep_kernel<<<gs, pdc::kSweepTile, 0, st>>>(w->W, L, sc);
         tb = L.temp_bytes;
-        CK(cub::DeviceRadixSort::SortKeys(L.temp, tb, L.pairs, L.pairs_s, (int)L.max_pairs, 0, 64, st),
+        CK(cub::DeviceRadixSort::SortKeys(L.temp, tb, L.pairs, L.pairs_s, (int)L.max_pairs, 0, 2 * L.bits, st),
            "sort pairs");
         pdc::large_narrow_kernel<<<gl, 256, 0, st>>>(w->W, L, sc, 0);
         tb = L.temp_bytes;
@@ -469,6 +548,7 @@ extern "C" int pdc_world_create(const pdc_config* cfg, int32_t n_scenes, const i
             L.nb_max = std::max(L.nb_max, body_offsets[sc + 1] - body_offsets[sc]);
         }
         L.max_pairs = std::max(1024LL, 64LL * L.nb_max);
+        for (L.bits = 1; L.bits < 31 && (1 << L.bits) < L.nb_max;) ++L.bits;
         size_t t1 = 0, t2 = 0, t3 = 0;
         cub::DeviceRadixSort::SortPairs(nullptr, t1, (unsigned int*)nullptr, (unsigned int*)nullptr, (int*)nullptr,
                                         (int*)nullptr, L.nb_max);
