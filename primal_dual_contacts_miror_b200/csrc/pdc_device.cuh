@@ -17,6 +17,11 @@ __device__ __forceinline__ double dot3(d3 a, d3 b) { return a.x * b.x + a.y * b.
 __device__ __forceinline__ d3 cross3(d3 a, d3 b) {
     return d3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
+// a x b with the first product of every component fused
+__device__ __forceinline__ d3 cross_rn(d3 a, d3 b) {
+    return d3{__fma_rn(a.y, b.z, -__dmul_rn(a.z, b.y)), __fma_rn(a.z, b.x, -__dmul_rn(a.x, b.z)),
+              __fma_rn(a.x, b.y, -__dmul_rn(a.y, b.x))};
+}
 __device__ __forceinline__ d3 ld3(const double* p) { return d3{p[0], p[1], p[2]}; }
 __device__ __forceinline__ void st3(double* p, d3 v) { p[0] = v.x; p[1] = v.y; p[2] = v.z; }
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }  // std::max
@@ -49,23 +54,27 @@ __device__ __forceinline__ d3 from_frame(const Frame& R, d3 f) {
 #define PDC_PERT 1e-16
 #define PDC_SQRT_PERT 1e-8
 #define PDC_SHIFT 1e-8
+// |f_t|^2, rounded the same way in every function of it
+__device__ __forceinline__ double cone_sq(double f1, double f2) {
+    return __dadd_rn(__dmul_rn(f1, f1), __dmul_rn(f2, f2));
+}
 __device__ __forceinline__ double cone_c(double fn, double f1, double f2, double mu) {
-    double r = f1 * f1 + f2 * f2 + PDC_PERT;
+    double r = cone_sq(f1, f2) + PDC_PERT;
     return sqrt(r) - mu * fn - PDC_SQRT_PERT - PDC_SHIFT;
 }
 __device__ __forceinline__ void cone_grad(double f1, double f2, double& g0, double& g1) {
-    double r = sqrt(f1 * f1 + f2 * f2 + PDC_PERT);
+    double r = sqrt(cone_sq(f1, f2) + PDC_PERT);
     g0 = f1 / r;
     g1 = f2 / r;
 }
 // Hessian (zz^T + p'I) r2^-3/2 with z = (f2, -f1), p' = 1e-6 (:23-35); packed (h00, h01, h11).
 __device__ __forceinline__ void cone_hess(double f1, double f2, double& h00, double& h01, double& h11) {
     const double p = 1e-6;
-    double r2 = f1 * f1 + f2 * f2 + p;
+    double r2 = cone_sq(f1, f2) + p;
     double r3 = pow(r2, -1.5);
-    h00 = (f2 * f2 + p) * r3;
+    h00 = __dadd_rn(__dmul_rn(f2, f2), p) * r3;
     h01 = (f2 * -f1) * r3;
-    h11 = (f1 * f1 + p) * r3;
+    h11 = __dadd_rn(__dmul_rn(f1, f1), p) * r3;
 }
 __device__ __forceinline__ double cone_radius(double fn, double mu) {
     double k = mu * fn + PDC_SQRT_PERT + PDC_SHIFT;
@@ -82,27 +91,43 @@ struct BlockReducer {
     double* slots;  // [2][N][32] in shared memory
     int parity;
     __device__ void init(double* s) { slots = s; parity = 0; }
+    // The warp stage halves the values with every exchange (lanes that differ in
+    // bit 4 keep one half of the values each, and so on), so M <= 8 sums take 9
+    // shuffles of doubles instead of 5 M, and M <= 16 take 17; then lane l adds
+    // the warps' slots of value l (both in the order of a plain shuffle tree).
     template <int M>
     __device__ __forceinline__ void sum(double (&v)[M]) {
-        static_assert(M <= N, "reduction wider than the slots");
+        static_assert(M <= N && M <= 16, "reduction wider than the slots");
+        constexpr int K = M <= 8 ? 8 : 16;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
         double* b = slots + parity * N * 32;
         parity ^= 1;
+        double x[K];
 #pragma unroll
-        for (int i = 0; i < M; ++i) {
-            double x = v[i];
+        for (int i = 0; i < K; ++i) x[i] = i < M ? v[i] : 0.0;
+        int idx = 0;  // value this lane ends up with
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-            if (lane == 0) b[i * 32 + warp] = x;
+        for (int h = K / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < h; ++i) {
+                const double mine = up ? x[i + h] : x[i];
+                const double send = up ? x[i] : x[i + h];
+                x[i] = mine + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+            if (up) idx += h;
         }
+        constexpr int left = K == 8 ? 2 : 1;  // lane bits not yet summed over
+#pragma unroll
+        for (int o = left; o >= 1; o >>= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+        if ((lane & (2 * left - 1)) == 0) b[warp * K + idx] = x[0];
         __syncthreads();
+        double t[8];  // at most 8 warps; the tree of a shuffle-down over the slots
 #pragma unroll
-        for (int i = 0; i < M; ++i) {
-            double x = (lane < nw) ? b[i * 32 + lane] : 0.0;
+        for (int w = 0; w < 8; ++w) t[w] = w < nw ? b[w * K + (lane & (K - 1))] : 0.0;
+        const double total = ((t[0] + t[4]) + (t[2] + t[6])) + ((t[1] + t[5]) + (t[3] + t[7]));
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-            v[i] = __shfl_sync(0xffffffffu, x, 0);
-        }
+        for (int i = 0; i < M; ++i) v[i] = __shfl_sync(0xffffffffu, total, i);
     }
     template <int M>
     __device__ __forceinline__ void max(double (&v)[M]) {
@@ -139,18 +164,15 @@ struct CtaTeam {
     int rank, size, slot;
     BlockReducer<16> red;
     int* s_int;  // shared: [0] carry, [1..32] warp partials
-    uint32_t* s_adj;  // shared: node adjacency of the symbolic factorisation
     unsigned int parity = 0;
-    __device__ CtaTeam(double* red_smem, int* int_smem, uint32_t* adj_smem) {
+    __device__ CtaTeam(double* red_smem, int* int_smem) {
         rank = threadIdx.x;
         size = blockDim.x;
         slot = blockIdx.x;
         red.init(red_smem);
         s_int = int_smem;
-        s_adj = adj_smem;
     }
     __device__ __forceinline__ void sync() { __syncthreads(); }
-    __device__ __forceinline__ uint32_t* adjacency(uint32_t*) const { return s_adj; }
     __device__ __forceinline__ bool any(bool p) { return __syncthreads_or(p) != 0; }
     // minimum over the team, one barrier (two alternating rows of warp slots)
     __device__ __forceinline__ unsigned min_u32(unsigned v) {
@@ -215,7 +237,6 @@ struct WarpTeam {
         slot = slot_;
     }
     __device__ __forceinline__ void sync() { __syncwarp(); }
-    __device__ __forceinline__ uint32_t* adjacency(uint32_t* scratch) const { return scratch; }
     __device__ __forceinline__ bool any(bool p) { return __any_sync(0xffffffffu, p) != 0; }
     __device__ __forceinline__ unsigned min_u32(unsigned v) {
         __syncwarp();  // a barrier, as the thread block's

@@ -57,6 +57,7 @@ struct EngineCfg {
 
 struct BatchPtrs {
     int n_scenes;
+    int smem_blocks; // factor blocks that fit each thread block's dynamic shared memory
     int grid_large;  // the host launches the grid kernel for scenes >= grid_min_bodies
     // single-scene launch (body_off == nullptr): sizes and step passed by value
     int single_nb, single_nc;
@@ -106,36 +107,18 @@ struct BatchPtrs {
     double* ru;    // 6
     double* pinv;  // 21
     double* dsc;   // 6  Jacobi scale 1/sqrt(diag A) of the iterative branch
-    // per-contact workspace
-    int* inc;       // 2 per contact
-    int* inc_o;     // 2 per contact: the incidence's other body (global index), -1 if static
-    int* islot;     // 2 per contact: incidence index of (contact, side), -1 for a static side
-    double* Xi;     // 3 per incidence: sigma X of its contact (sigma = -1 on side 0, +1 on side 1)
-    double* armI;   // 3 per incidence: the lever arm of its side
-    double* f;      // 3
-    double* lam;    // 2
-    double* fT;     // 3
-    double* lT;     // 2
-    double* Xi2;    // 6: the second line-search trial of a pair (Xi, fT, lT of step / 2)
-    double* fT2;    // 3
-    double* lT2;    // 2
-    double* df;     // 3
-    double* dl;     // 2
-    double* rf;     // 3
-    double* rl;     // 2
-    double* kn;     // 1 (m_nonSmoothK normal slot)
-    double* cv;     // 2 constraint values
-    double* gr;     // 2 gradients
-    double* hs;     // 3 hessian (packed)
-    double* tq;     // 3: tangential-weight form T_t^T M^-1 T_t of both bodies (packed 2x2)
-    double* wu;     // 3: relative velocity J u at the iterate (line-search base)
-    double* wd;     // 3: J du of the search direction
-    double* invC;   // 2
-    double* knInv;  // 1
-    double* ktInv;  // 3 (packed symmetric inverse of K_t)
-    double* sf;     // 3
-    double* X;      // 3 world vector gathered by bodies
-    double* W;      // 6 R K^-1 R^T packed (xx,yy,zz,xy,xz,yz)
+    // incidences of active bodies, in contact order per body, 2 per contact
+    int* inc;       // contact << 1 | side
+    int* inc_o;     // the other body (global index), -1 if static; the block and
+                    // warp teams' factor keeps the block it adds to here
+    int* inc_g;     // the incidences (slots) of each factor block, block by block
+    int* islot;     // incidence index of (contact, side), -1 for a static side
+    double* it;     // tiles of 32 incidences, kIncFields runs of 32 values each
+    double* ct;     // tiles of 32 contacts, kFields runs of 32 values each
+    // 12 side by side per incidence, for the body phases that read all of them:
+    // W = R K^-1 R^T of its contact, packed (xx,yy,zz,xy,xz,yz), the lever arm of
+    // its side, the lever arm of the other side
+    double* G;
     // mixed precision (FP32 inner PCG): per-contact W and X, per-body vectors
     float* Wf;     // 6 per contact
     float* Xf;     // 3 per contact
@@ -162,6 +145,44 @@ struct BatchPtrs {
 
 #define PDC_STATUS_BAD_INPUT 16
 
+// Per-contact workspace: tiles of 32 contacts, one run of 32 values per field, so
+// that a warp's loads and stores are coalesced and every field of a contact is
+// a constant offset from one address.  (With a contact's components side by
+// side, each of the ~60 loads per contact and phase touched up to 32 lines per
+// warp, and the load-store unit bound the contact phases: 39 us per residual
+// pass over 1,536 contacts; with one plane per component over the whole batch
+// the ~60 addresses cost 3,900 bytes of register spills.)
+enum ContactField {
+    F_frame = 0,          // 9: copy of the input
+    F_arm = 9,            // 6: lever arms of both sides (copy of the input)
+    F_f = 15,             // 3
+    F_lam = 18,           // 2
+    F_fT = 20,            // 3: line-search trial, then 2: its multipliers
+    F_lT = 23,
+    F_fT2 = 25,           // the second trial of a pair
+    F_lT2 = 28,
+    F_df = 30,            // 3
+    F_dl = 33,            // 2
+    F_rf = 35,            // 3
+    F_rl = 38,            // 2
+    F_kn = 40,            // 1 (m_nonSmoothK normal slot)
+    F_cv = 41,            // 2 constraint values
+    F_gr = 43,            // 2 gradients
+    F_hs = 45,            // 3 hessian (packed)
+    F_tq = 48,            // 3: tangential-weight form T_t^T M^-1 T_t of both bodies (packed 2x2)
+    F_wu = 51,            // 3: relative velocity J u at the iterate (line-search base)
+    F_wd = 54,            // 3: J du of the search direction
+    F_invC = 57,          // 2
+    F_knInv = 59,         // 1
+    F_ktInv = 60,         // 3 (packed symmetric inverse of K_t)
+    F_sf = 63,            // 3
+    kFields = 66
+};
+// Per-incidence workspace, in tiles of 32 likewise: sigma X of its contact (sigma
+// = -1 on side 0, +1 on side 1), the lever arm of its side, and the X of the
+// second line-search trial of a pair.
+enum IncField { I_X = 0, I_arm = 3, I_X2 = 6, kIncFields = 9 };
+
 // sparse direct solve: nodes per scene (bitset width)
 constexpr int kSparseMax = 256;
 constexpr int kSparseWords = kSparseMax / 32;
@@ -171,13 +192,18 @@ constexpr int kSparseWords = kSparseMax / 32;
 constexpr int kRowCap = kSparseMax * (kSparseMax - 1) / 2;
 // 6x6 blocks of a factor: the off-diagonal ones and a diagonal one per node
 constexpr int kBlockCap = kRowCap + kSparseMax;
-// doubles of a packed inverse diagonal factor, padded to a multiple of 16 bytes
-constexpr int kInvStride = 22;
-// bytes of a slot before its blocks (bitsets, index arrays, inverse diagonal
-// factors and node vectors; the layout of SceneSolver::direct_ws)
-constexpr long long kSparseHeaderBytes = 4LL * (3LL * kSparseMax * kSparseWords + 13LL * (kSparseMax + 8) +
-                                                kBlockCap + 8) +
-                                         2LL * kBlockCap + 8LL * (kInvStride + 2 * 6 + 36) * kSparseMax;
+// bytes of a slot before its blocks (bitsets, index arrays, block descriptors
+// and the node vector; the layout of SceneSolver::direct_ws), plus the diagonal
+// blocks and two spare ones (a zero block and room to read past the last)
+constexpr long long kSparseHeaderBytes = 4LL * (3LL * kSparseMax * kSparseWords + 12LL * (kSparseMax + 8)) +
+                                         16LL * (kBlockCap + 2) +
+                                         8LL * (6 * (kSparseMax + 2) + 36 * (kSparseMax + 2));
+// Levels whose update lists (column patterns) have at most this many entries
+// are updated by a thread per row (substituted backward entry by entry).
+constexpr int kShortList = 4;
+// Dynamic shared memory of a thread block of the batched kernel: the node vector,
+// then factor blocks (the adjacency bitsets while ordering).
+constexpr int kSmemVector = 6 * (kSparseMax + 2);
 
 // The large-scene teams (whole GPU, one cluster) solve one scene per launch and
 // factor up to kSparseMaxLarge active bodies: the whole direct branch, which
@@ -260,6 +286,7 @@ class SceneSolver {
     int n_local, n_active;
     bool dense_mode;
     int sp_nw;  // bitset words in use (large teams)
+    bool in_smem = false;  // the factor's blocks are in shared memory, not in the team's slot
     int status;
     // sparse-factor capacities: the large-scene teams run one scene per launch
     static constexpr bool kLargeTeam = Team::kind >= 2;
@@ -311,19 +338,57 @@ class SceneSolver {
         return C.mu;
     }
 
-    // Gather sum over the incidences of body gb of sigma * [X; c x X]: the
-    // contacts left sigma X in the body's own incidence slots (put_x), so the
-    // loads are contiguous and independent of each other
-    __device__ __forceinline__ void gather(int gb, double out[6], const double* xbuf = nullptr) const {
+    // fields of contact gc / of an incidence slot (kFields and kIncFields runs of 32)
+    __device__ __forceinline__ double* contact(int gc) const {
+        return B.ct + (long long)(gc >> 5) * (32 * kFields) + (gc & 31);
+    }
+    __device__ __forceinline__ double* incidence(int slot) const {
+        return B.it + (long long)(slot >> 5) * (32 * kIncFields) + (slot & 31);
+    }
+    __device__ __forceinline__ static d3 fld3(const double* P, int f) {
+        return d3{P[32 * f], P[32 * f + 32], P[32 * f + 64]};
+    }
+    __device__ __forceinline__ static void fst3(double* P, int f, d3 v) {
+        P[32 * f] = v.x;
+        P[32 * f + 32] = v.y;
+        P[32 * f + 64] = v.z;
+    }
+    __device__ __forceinline__ static Frame frame(const double* P) {
+        Frame f;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) f.m[i] = P[32 * (F_frame + i)];
+        return f;
+    }
+    __device__ __forceinline__ static d3 arm(const double* P, int side) { return fld3(P, F_arm + 3 * side); }
+    __device__ __forceinline__ static void ld6(const double* p, double* v) {  // 16-byte aligned
+        const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1],
+                      c = reinterpret_cast<const double2*>(p)[2];
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y;
+    }
+    __device__ __forceinline__ static void st6(double* p, const double* v) {
+        reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
+        reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
+        reinterpret_cast<double2*>(p)[2] = make_double2(v[4], v[5]);
+    }
+    // W (packed), own and other lever arm of an incidence
+    __device__ __forceinline__ void ldg12(int slot, double* v) const {
+        ld6(B.G + 12LL * slot, v);
+        ld6(B.G + 12LL * slot + 6, v + 6);
+    }
+
+    // Gather sum over the incidences of body gb of sigma * [X; c x X], in incidence
+    // order: the contacts left sigma X in the body's own incidence slots (put_x),
+    // so the loads are independent of each other.  (Lanes splitting a body's
+    // incidences change the order of the sums, and with it the rounding that an
+    // unloaded symmetric stack amplifies.)
+    __device__ __forceinline__ void gather(int gb, double out[6], int xf = I_X) const {
         const int st = B.inc_start[gb], n = B.inc_cnt[gb];
-        const double* xi = (xbuf ? xbuf : B.Xi) + 3LL * st;
-        const double* ai = B.armI + 3LL * st;
         double a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0;
 #pragma unroll 4
         for (int k = 0; k < n; ++k) {
-            const d3 x = ld3(xi + 3 * k);
-            const d3 arm = ld3(ai + 3 * k);
-            const d3 t = cross3(arm, x);
+            const double* Q = incidence(st + k);
+            const d3 x = fld3(Q, xf);
+            const d3 t = cross3(fld3(Q, I_arm), x);
             a0 += x.x; a1 += x.y; a2 += x.z;
             a3 += t.x; a4 += t.y; a5 += t.z;
         }
@@ -331,11 +396,11 @@ class SceneSolver {
     }
     // Contact gc's world vector X into the incidence slots of its two sides, with
     // the side's sign (-X for side 0, X for side 1; static sides have no slot)
-    __device__ __forceinline__ void put_x(int gc, d3 x, double* xbuf = nullptr) const {
-        const int s0 = B.islot[2 * gc], s1 = B.islot[2 * gc + 1];
-        double* xo = xbuf ? xbuf : B.Xi;
-        if (s0 >= 0) st3(xo + 3LL * s0, scl3(-1.0, x));
-        if (s1 >= 0) st3(xo + 3LL * s1, x);
+    // -- field xf of the slots
+    __device__ __forceinline__ void put_x(int gc, d3 x, int xf = I_X) const {
+        const int2 sl = reinterpret_cast<const int2*>(B.islot)[gc];
+        if (sl.x >= 0) fst3(incidence(sl.x), xf, scl3(-1.0, x));
+        if (sl.y >= 0) fst3(incidence(sl.y), xf, x);
     }
     // (M / charMass) v  for an active body
     __device__ __forceinline__ void mass_mul(int gb, const double* v, double* y) const {
@@ -405,7 +470,12 @@ class SceneSolver {
         // per-contact speeds for nonDimensionalParams (:38-63): velExt = v (+ g dt if active)
         for (int c = tid; c < nc; c += nt) {
             const int gc = c0 + c;
+            double* const P = contact(gc);
             const Frame R = ld_frame(B.frame + 9 * gc);
+#pragma unroll
+            for (int k = 0; k < 9; ++k) P[32 * (F_frame + k)] = R.m[k];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) P[32 * (F_arm + k)] = B.arm[6 * gc + k];
             d3 half[2];
             bool hasStatic = false;
             for (int j = 0; j < 2; ++j) {
@@ -416,7 +486,7 @@ class SceneSolver {
                     ve[3 + r] = B.ang[3 * gb + r];
                 }
                 if (!B.is_static[gb]) {
-                    for (int r = 0; r < 3; ++r) ve[r] += g[r] * dt;
+                    for (int r = 0; r < 3; ++r) ve[r] = fma(g[r], dt, ve[r]);
                 } else {
                     hasStatic = true;
                 }
@@ -430,7 +500,7 @@ class SceneSolver {
             for (int j = 0; j < 2; ++j) {
                 double sp = sqrt(dot3(half[j], half[j]));
                 if (hasStatic) sp = dmax(sp, nrel);
-                B.X[3 * gc + j] = sp;
+                P[32 * (F_wu + j)] = sp;
             }
         }
         T.sync();
@@ -454,11 +524,15 @@ class SceneSolver {
             double spd = 0;
             for (int k = 0; k < n; ++k) {
                 const int e = B.inc[st + k];
-                spd = dmax(spd, B.X[3 * (e >> 1) + (e & 1)]);
+                spd = dmax(spd, contact(e >> 1)[32 * (F_wu + (e & 1))]);
                 const int go = b0 + B.cbody[2 * (e >> 1) + 1 - (e & 1)];
                 B.inc_o[st + k] = B.is_static[go] ? -1 : go;
                 B.islot[e] = st + k;  // e = 2 gc + side
-                st3(B.armI + 3LL * (st + k), ld3(B.arm + 6 * (e >> 1) + 3 * (e & 1)));
+                const double* P = contact(e >> 1);
+                const d3 own = arm(P, e & 1), oth = arm(P, 1 - (e & 1));
+                fst3(incidence(st + k), I_arm, own);
+                const double a[6] = {own.x, own.y, own.z, oth.x, oth.y, oth.z};
+                st6(B.G + 12LL * (st + k) + 6, a);
             }
             const double m = B.mass[gb];
             const double* I = B.inertia + 6 * gb;
@@ -503,13 +577,15 @@ class SceneSolver {
             for (int r = 0; r < 3; ++r) {
                 double v = B.vel[3 * gb + r], w = B.ang[3 * gb + r];
                 double vo = v;
-                if (!B.is_static[gb]) vo += g[r] * dt;
+                if (!B.is_static[gb]) vo += __dmul_rn(g[r], dt);
                 B.u[6 * gb + r] = v / cs;
                 B.u[6 * gb + 3 + r] = w / cs;
                 B.uold[6 * gb + r] = vo / cs;
                 B.uold[6 * gb + 3 + r] = w / cs;
                 B.du[6 * gb + r] = 0;
                 B.du[6 * gb + 3 + r] = 0;
+                B.ru[6 * gb + r] = 0;  // static rows stay zero (calculateResiduals :151-163)
+                B.ru[6 * gb + 3 + r] = 0;
             }
         }
         // preprocess (NonSmoothContactForce.cpp:8-48) + initForces (:49-52)
@@ -521,22 +597,23 @@ class SceneSolver {
         T.sync();
         for (int c = tid; c < nc; c += nt) {
             const int gc = c0 + c;
+            double* const P = contact(gc);
             double k = 0;
             if (C.spring_based) {
                 k += -reduction * B.depth[gc] / dt / cs;
             } else {
-                d3 w = rel_vel(gc, B.u);
+                d3 w = rel_vel(gc, P, B.u);
                 k += w.x * C.restitution;
             }
-            B.kn[gc] = k;
+            P[32 * F_kn] = k;
             {  // calculateTangentialWeight's mass term as a 2x2 form in the tangent direction
-                const Frame R = ld_frame(B.frame + 9 * gc);
+                const Frame R = frame(P);
                 const d3 t1 = from_frame(R, d3{0.0, 1.0, 0.0}), t2 = from_frame(R, d3{0.0, 0.0, 1.0});
                 double q00 = 0, q01 = 0, q11 = 0;
                 for (int j = 0; j < 2; ++j) {
                     const int gb = b0 + B.cbody[2 * gc + j];
                     if (B.is_static[gb]) continue;
-                    const d3 c = ld3(B.arm + 6 * gc + 3 * j);
+                    const d3 c = arm(P, j);
                     const d3 a = cross3(c, t1), e = cross3(c, t2);
                     const double im = 1.0 / B.mass[gb];
                     const double* J = B.inv_inertia + 6 * gb;
@@ -548,15 +625,11 @@ class SceneSolver {
                     q01 += im * dot3(t1, t2) + dot3(a, Je);
                     q11 += im * dot3(t2, t2) + dot3(e, Je);
                 }
-                B.tq[3 * gc] = q00;
-                B.tq[3 * gc + 1] = q01;
-                B.tq[3 * gc + 2] = q11;
+                fst3(P, F_tq, d3{q00, q01, q11});
             }
-            B.f[3 * gc] = 1;
-            B.f[3 * gc + 1] = 0;
-            B.f[3 * gc + 2] = 0;
-            B.lam[2 * gc] = 1e-2;
-            B.lam[2 * gc + 1] = C.only_normal ? 0.0 : 1e-2;  // only_normal: lambda_t absent
+            fst3(P, F_f, d3{1.0, 0.0, 0.0});
+            P[32 * F_lam] = 1e-2;
+            P[32 * (F_lam + 1)] = C.only_normal ? 0.0 : 1e-2;  // only_normal: lambda_t absent
         }
         T.sync();
         return true;
@@ -564,106 +637,107 @@ class SceneSolver {
 
     // toLocal(vels) = -T0^T u0 - T1^T u1 = R^T[(v1 + w1 x c1) - (v0 + w0 x c0)]
     // (ContactInfo.h:46-51); non-local/static bodies read their (fixed) u.
-    __device__ __forceinline__ d3 rel_vel(int gc, const double* uvec) const {
-        const Frame R = ld_frame(B.frame + 9 * gc);
+    __device__ __forceinline__ d3 rel_vel(int gc, const double* P, const double* uvec) const {
         const int gb0 = b0 + B.cbody[2 * gc], gb1 = b0 + B.cbody[2 * gc + 1];
-        d3 p0 = point_vel(uvec + 6 * gb0, ld3(B.arm + 6 * gc));
-        d3 p1 = point_vel(uvec + 6 * gb1, ld3(B.arm + 6 * gc + 3));
-        return to_frame(R, sub3(p1, p0));
+        double u0[6], u1[6];
+        ld6(uvec + 6LL * gb0, u0);
+        ld6(uvec + 6LL * gb1, u1);
+        return to_frame(frame(P), sub3(point_vel(u1, arm(P, 1)), point_vel(u0, arm(P, 0))));
     }
 
     // Tangential weight (calculateTangentialWeight, NonSmoothContactForce.cpp:74-104)
     // The direction d = R (0, th0, th1) enters as hh_j = s_j [d; c_j x d], so the
     // sum over the active bodies of hh_j^T M_j^-1 hh_j is th^T Q th with the
     // per-contact Q = sum_j T_j,t^T M_j^-1 T_j,t computed once per solve (tq).
-    __device__ __forceinline__ double tangential_weight(int gc, const Frame& R, d3 w, double fn) const {
-        (void)R;
+    __device__ __forceinline__ double tangential_weight(const double* P, d3 w, double rad) const {
         const double tn = sqrt(w.y * w.y + w.z * w.z);
         double th0 = w.y, th1 = w.z;
         if (tn > 0) { th0 = w.y / tn; th1 = w.z / tn; }
-        const double* Q = B.tq + 3 * gc;
-        const double fw = (Q[0] * th0 * th0 + 2.0 * Q[1] * th0 * th1 + Q[2] * th1 * th1) * cm;
-        const double rad = cone_radius(fn, cmu(gc));
+        const d3 Q = fld3(P, F_tq);
+        const double fw = (Q.x * th0 * th0 + 2.0 * Q.y * th0 * th1 + Q.z * th1 * th1) * cm;
         return dmin(rad / (tn + 1e-8) * fw, 1.0);
     }
 
     // OnlyNormalForce residuals (OnlyNormalForce.cpp:46-89) and AC term (:202-217):
     // rf = -w_n (- compliance f_n) + lambda - k, rl = lambda (-f_n) + mu_c, unit
     // weight, AC = max(f_n - (w_n + k + spring f_n), 0) - f_n; X = -R (f_n, 0, 0).
-    __device__ __forceinline__ void normal_residual(int gc, const Frame& R, d3 w, double fn, double ln, double muc,
-                                                    double* rfo, double* rlo, double& wrf2, double& rl2,
-                                                    double& ac2, double* xbuf = nullptr) const {
+    __device__ __forceinline__ void normal_residual(int gc, const double* P, const Frame& R, d3 w, double fn,
+                                                    double ln, double muc, d3& rfo, double& rl0, double& wrf2,
+                                                    double& rl2, double& ac2, int xf) const {
+        const double kn = P[32 * F_kn];
         double r0 = 0 - w.x;
         if (C.spring_based) r0 -= compliance * cm * fn;
         r0 += ln;
-        r0 -= B.kn[gc];
-        const double rl0 = ln * (-fn) + muc;
+        r0 -= kn;
+        rl0 = ln * (-fn) + muc;
         wrf2 += r0 * r0;
         rl2 += rl0 * rl0;
-        const double tp = fn - (w.x + B.kn[gc] + spring_term * fn);
+        const double tp = fn - (w.x + kn + spring_term * fn);
         const double a0 = dmax(tp, 0.0) - fn;
         ac2 += a0 * a0;
-        if (rfo) { rfo[0] = r0; rfo[1] = 0; rfo[2] = 0; }
-        if (rlo) { rlo[0] = rl0; rlo[1] = 0; }
-        put_x(gc, scl3(-1.0, from_frame(R, d3{fn, 0.0, 0.0})), xbuf);
+        rfo = d3{r0, 0.0, 0.0};
+        put_x(gc, scl3(-1.0, from_frame(R, d3{fn, 0.0, 0.0})), xf);
     }
 
-    // Residuals of one contact at the current iterate with its constraint values
-    // and gradient just computed (nonSmoothResiduals :119-172, ACVector :53-73),
-    // before the centering term is known: adds |wrf|^2, (lambda . c)^2 per
-    // constraint and |AC|^2; writes rf and X = -R f.
-    __device__ __forceinline__ void contact_residual_c(int gc, const double* uvec, const double* fv, double l0,
-                                                       double l1, double cn, double cc, double g0, double g1,
-                                                       double* rf_out, double& wrf2, double& a2, double& ac2) const {
-        const Frame R = ld_frame(B.frame + 9 * gc);
-        const d3 w = rel_vel(gc, uvec);
-        st3(B.wu + 3 * gc, w);  // the line search steps from here: J(u + a du) = J u + a J du
-        const double fn = fv[0];
-        if (C.only_normal) {
-            double rl2 = 0;
-            normal_residual(gc, R, w, fn, l0, 0.0, rf_out, nullptr, wrf2, rl2, ac2);
-            a2 += rl2;
-            return;
-        }
-        const double f1 = fv[1], f2 = fv[2];
-        const double mu = cmu(gc);
+    // Residuals of one contact (nonSmoothResiduals :119-172, ACVector :53-73) at
+    // force fv and multiplier l1 with relative velocity w and cone gradient (g0,
+    // g1): rf, its weighted square and |AC|^2; X = -R f into the incidence slots.
+    __device__ __forceinline__ d3 cone_residual(int gc, const double* P, const Frame& R, d3 w, d3 fv, double l0,
+                                                double l1, double g0, double g1, double mu, double& wrf2, double& ac2,
+                                                int xf) const {
+        const double kn = P[32 * F_kn], fn = fv.x;
         double r0 = 0 - w.x, r1 = 0 - w.y, r2 = 0 - w.z;
         if (C.spring_based) r0 -= compliance * cm * fn;
         r0 += l0;
         r1 -= l1 * g0;
         r2 -= l1 * g1;
-        r0 -= B.kn[gc];
-        const double a0 = l0 * cn, a1 = l1 * cc;
-        const double wt = tangential_weight(gc, R, w, fn);
+        r0 -= kn;
+        const double rad = cone_radius(fn, mu);
+        const double wt = tangential_weight(P, w, rad);
         const double w1 = r1 * wt, w2 = r2 * wt;
         wrf2 += r0 * r0 + w1 * w1 + w2 * w2;
-        a2 += a0 * a0 + a1 * a1;
         // Alart-Curnier (:60-70)
-        const double tp = fn - (w.x + B.kn[gc] + spring_term * fn);
+        const double tp = fn - (w.x + kn + spring_term * fn);
         const double q0 = dmax(tp, 0.0) - fn;
-        const double rad = cone_radius(fn, mu);
-        const double td0 = f1 - w.y, td1 = f2 - w.z;
+        const double td0 = fv.y - w.y, td1 = fv.z - w.z;
         const double tdn = sqrt(td0 * td0 + td1 * td1);
         double p0 = td0, p1 = td1;
         if (!(tdn < rad)) { p0 = td0 * rad / tdn; p1 = td1 * rad / tdn; }
-        const double q1 = p0 - f1, q2 = p1 - f2;
+        const double q1 = p0 - fv.y, q2 = p1 - fv.z;
         ac2 += q0 * q0 + q1 * q1 + q2 * q2;
-        rf_out[0] = r0; rf_out[1] = r1; rf_out[2] = r2;
-        put_x(gc, scl3(-1.0, from_frame(R, d3{fn, f1, f2})));
+        put_x(gc, scl3(-1.0, from_frame(R, fv)), xf);
+        return d3{r0, r1, r2};
     }
 
-    // ru = M(u - uold) (+ gather of T_j f); static rows zero (calculateResiduals :151-163)
-    __device__ __forceinline__ void body_residual(int gb, const double* ub, double* ru_out, double& ru2,
-                                                  const double* xbuf = nullptr) const {
-        double d[6], y[6], gth[6];
-        for (int r = 0; r < 6; ++r) d[r] = ub[r] - B.uold[6 * gb + r];
-        mass_mul(gb, d, y);
-        gather(gb, gth, xbuf);
-        for (int r = 0; r < 6; ++r) {
-            const double v = y[r] + gth[r];
-            ru2 += v * v;
-            if (ru_out) ru_out[r] = v;
+    // Residuals of one contact at the current iterate with its constraint values
+    // and gradient just computed, before the centering term is known: adds
+    // |wrf|^2, (lambda . c)^2 per constraint and |AC|^2; writes rf and X = -R f.
+    __device__ __forceinline__ void contact_residual_c(int gc, double* P, d3 fv, double l0, double l1, double cn, double cc1,
+                                                       double g0, double g1, double mu, double& wrf2, double& a2,
+                                                       double& ac2) const {
+        const d3 w = rel_vel(gc, P, B.u);
+        fst3(P, F_wu, w);  // the line search steps from here: J(u + a du) = J u + a J du
+        const Frame R = frame(P);
+        d3 r;
+        if (C.only_normal) {
+            double rl0;
+            normal_residual(gc, P, R, w, fv.x, l0, 0.0, r, rl0, wrf2, a2, ac2, I_X);
+        } else {
+            const double a0 = l0 * cn, a1 = l1 * cc1;
+            a2 += a0 * a0 + a1 * a1;
+            r = cone_residual(gc, P, R, w, fv, l0, l1, g0, g1, mu, wrf2, ac2, I_X);
         }
+        fst3(P, F_rf, r);
+    }
+
+    // ru = M(u - uold) (+ gather of T_j f) of one active body (calculateResiduals :151-163)
+    __device__ __forceinline__ void body_residual(int gb, const double* ub, int xf, double* v) const {
+        double gth[6], d[6], y[6];
+        ld6(B.uold + 6LL * gb, d);
+        for (int r = 0; r < 6; ++r) d[r] = ub[r] - d[r];
+        mass_mul(gb, d, y);
+        gather(gb, gth, xf);
+        for (int r = 0; r < 6; ++r) v[r] = y[r] + gth[r];
     }
 
     // ------------------------------------------------------------ Newton
@@ -686,34 +760,36 @@ class SceneSolver {
             double e[5] = {0, 0, 0, 0, 0};  // ru2, wrf2, sum a^2, ac2, sum a
             for (int c = tid; c < nc; c += nt) {
                 const int gc = c0 + c;
-                const double fn = B.f[3 * gc], f1 = B.f[3 * gc + 1], f2 = B.f[3 * gc + 2];
-                const double cn = -fn;
-                double cc = 0, g0 = 0, g1 = 0, h0 = 0, h1 = 0, h2 = 0;  // only_normal: c = -f_n alone
+                double* const P = contact(gc);
+                const d3 fv = fld3(P, F_f);
+                const double cn = -fv.x;
+                double cc1 = 0, mu = 0;  // only_normal: c = -f_n alone
+                d3 h = d3{0.0, 0.0, 0.0};
+                double g0 = 0, g1 = 0;
                 if (!C.only_normal) {
-                    cc = cone_c(fn, f1, f2, cmu(gc));
-                    cone_grad(f1, f2, g0, g1);
-                    cone_hess(f1, f2, h0, h1, h2);
+                    mu = cmu(gc);
+                    cc1 = cone_c(fv.x, fv.y, fv.z, mu);
+                    cone_grad(fv.y, fv.z, g0, g1);
+                    cone_hess(fv.y, fv.z, h.x, h.y, h.z);
                 }
-                B.cv[2 * gc] = cn;
-                B.cv[2 * gc + 1] = cc;
-                B.gr[2 * gc] = g0;
-                B.gr[2 * gc + 1] = g1;
-                B.hs[3 * gc] = h0;
-                B.hs[3 * gc + 1] = h1;
-                B.hs[3 * gc + 2] = h2;
-                const double l0 = B.lam[2 * gc], l1 = B.lam[2 * gc + 1];
-                e[4] += l0 * cn + l1 * cc;
-                contact_residual_c(gc, B.u, B.f + 3 * gc, l0, l1, cn, cc, g0, g1, B.rf + 3 * gc, e[1], e[2], e[3]);
+                P[32 * F_cv] = cn;
+                P[32 * (F_cv + 1)] = cc1;
+                P[32 * F_gr] = g0;
+                P[32 * (F_gr + 1)] = g1;
+                fst3(P, F_hs, h);
+                const double l0 = P[32 * F_lam], l1 = P[32 * (F_lam + 1)];
+                e[4] += __fma_rn(l0, cn, __dmul_rn(l1, cc1));
+                contact_residual_c(gc, P, fv, l0, l1, cn, cc1, g0, g1, mu, e[1], e[2], e[3]);
             }
             T.sync();
             for (int i = tid; i < n_local; i += nt) {
                 const int gb = B.lbody[b0 + i];
-                if (!B.local[gb]) continue;
-                if (B.is_static[gb]) {
-                    for (int r = 0; r < 6; ++r) B.ru[6 * gb + r] = 0;
-                    continue;
-                }
-                body_residual(gb, B.u + 6 * gb, B.ru + 6 * gb, e[0]);
+                if (!active(gb)) continue;
+                double ub[6], v[6];
+                ld6(B.u + 6LL * gb, ub);
+                body_residual(gb, ub, I_X, v);
+                st6(B.ru + 6LL * gb, v);
+                for (int r = 0; r < 6; ++r) e[0] += v[r] * v[r];
             }
             T.sum(e);
             const double sDualGap = -(e[4] / n_cons);
@@ -732,44 +808,46 @@ class SceneSolver {
             // linsysAddition (:173-253): per-contact K, K^-1, sf, W, rhs vector
             for (int c = tid; c < nc; c += nt) {
                 const int gc = c0 + c;
-                const double ln = B.lam[2 * gc], lt = B.lam[2 * gc + 1];
+                double* const P = contact(gc);
+                const double ln = P[32 * F_lam], lt = P[32 * (F_lam + 1)];
+                const double cv0 = P[32 * F_cv], cv1 = P[32 * (F_cv + 1)];
                 // only_normal regularises c - eps (OnlyNormalForce.cpp:104), not c - eps lambda
-                const double ic0 = 1. / (B.cv[2 * gc] - eps * (C.only_normal ? 1.0 : ln));
-                const double ic1 = C.only_normal ? 0.0 : 1. / (B.cv[2 * gc + 1] - eps * lt);
-                B.invC[2 * gc] = ic0;
-                B.invC[2 * gc + 1] = ic1;
-                const double g0 = B.gr[2 * gc], g1 = B.gr[2 * gc + 1];
+                const double ic0 = 1. / (cv0 - eps * (C.only_normal ? 1.0 : ln));
+                const double ic1 = C.only_normal ? 0.0 : 1. / (cv1 - eps * lt);
+                P[32 * F_invC] = ic0;
+                P[32 * (F_invC + 1)] = ic1;
+                const double g0 = P[32 * F_gr], g1 = P[32 * (F_gr + 1)];
                 double lNorm = -ln * ic0;
                 if (C.spring_based) lNorm += compliance * cm;
                 // rl = lambda c + mu_c (nonSmoothResiduals :150-170), kept for the
                 // force recovery and the gradient-descent fallback
-                const double rl0 = ln * B.cv[2 * gc] + muc;
-                const double rl1 = C.only_normal ? 0.0 : lt * B.cv[2 * gc + 1] + muc;
-                B.rl[2 * gc] = rl0;
-                B.rl[2 * gc + 1] = rl1;
+                const double rl0 = ln * cv0 + muc;
+                const double rl1 = C.only_normal ? 0.0 : lt * cv1 + muc;
+                P[32 * F_rl] = rl0;
+                P[32 * (F_rl + 1)] = rl1;
                 const double a = -lt * ic1;
-                const double sf0 = B.rf[3 * gc] + (-rl0 * ic0);
-                const double sf1 = B.rf[3 * gc + 1] + g0 * rl1 * ic1;
-                const double sf2 = B.rf[3 * gc + 2] + g1 * rl1 * ic1;
-                B.sf[3 * gc] = sf0;
-                B.sf[3 * gc + 1] = sf1;
-                B.sf[3 * gc + 2] = sf2;
+                const d3 rf = fld3(P, F_rf);
+                const d3 sf = d3{rf.x + (-rl0 * ic0), rf.y + g0 * rl1 * ic1, rf.z + g1 * rl1 * ic1};
+                fst3(P, F_sf, sf);
                 const double kni = 1. / (eps + lNorm);
-                B.knInv[gc] = kni;
-                const double k00 = eps + a * g0 * g0 + lt * B.hs[3 * gc];
-                const double k01 = 0 + a * g0 * g1 + lt * B.hs[3 * gc + 1];
-                const double k11 = eps + a * g1 * g1 + lt * B.hs[3 * gc + 2];
+                P[32 * F_knInv] = kni;
+                const d3 h = fld3(P, F_hs);
+                const double k00 = eps + a * g0 * g0 + lt * h.x;
+                const double k01 = 0 + a * g0 * g1 + lt * h.y;
+                const double k11 = eps + a * g1 * g1 + lt * h.z;
                 const double det = k00 * k11 - k01 * k01;
                 double t00 = k11 / det, t01 = -k01 / det, t11 = k00 / det;
                 if (C.only_normal) t00 = t01 = t11 = 0;  // no tangential block
-                B.ktInv[3 * gc] = t00;
-                B.ktInv[3 * gc + 1] = t01;
-                B.ktInv[3 * gc + 2] = t11;
-                const Frame R = ld_frame(B.frame + 9 * gc);
-                frame_sandwich(R, kni, t00, t01, t11, B.W + 6 * gc);
+                fst3(P, F_ktInv, d3{t00, t01, t11});
+                const Frame R = frame(P);
+                double W[6];
+                frame_sandwich(R, kni, t00, t01, t11, W);
+                const int2 sl = reinterpret_cast<const int2*>(B.islot)[gc];
+                if (sl.x >= 0) st6(B.G + 12LL * sl.x, W);
+                if (sl.y >= 0) st6(B.G + 12LL * sl.y, W);
                 if (C.mixed)
-                    for (int q = 0; q < 6; ++q) B.Wf[6 * gc + q] = (float)B.W[6 * gc + q];
-                const d3 ks = d3{sf0 * kni, t00 * sf1 + t01 * sf2, t01 * sf1 + t11 * sf2};
+                    for (int q = 0; q < 6; ++q) B.Wf[6 * gc + q] = (float)W[q];
+                const d3 ks = d3{sf.x * kni, t00 * sf.y + t01 * sf.z, t01 * sf.y + t11 * sf.z};
                 put_x(gc, from_frame(R, ks));
             }
             T.sync();
@@ -777,7 +855,10 @@ class SceneSolver {
             double rr[3] = {0, 0, 0};  // r.z, b.b, |D b|^2 (iterative branch)
             const bool rows_mode = !kLargeTeam && dense_mode;
             if constexpr (!kLargeTeam) {
-                if (dense_mode) assemble_rows(eps);
+                if (dense_mode) {
+                    if (Team::kind == 0 && in_smem) assemble_rows<Team::kind == 0>(eps);
+                    else assemble_rows<false>(eps);
+                }
             }
             for (int i = rows_mode ? n_local : tid; i < n_local; i += nt) {
                 const int gb = B.lbody[b0 + i];
@@ -804,17 +885,22 @@ class SceneSolver {
                 }
                 const int st0 = B.inc_start[gb], n = B.inc_cnt[gb];
                 for (int k = 0; k < n; ++k) {
-                    const int e2 = B.inc[st0 + k];
-                    const int gc = e2 >> 1, side = e2 & 1;
-                    const double* W = B.W + 6 * gc;
-                    const d3 c = ld3(B.arm + 6 * gc + 3 * side);
+                    double W[12];
+                    ldg12(st0 + k, W);
+                    const d3 c = ld3(W + 6);
                     // Y = C W (C = [c]x): column k of Y = c x W_col_k
                     const d3 wc0 = d3{W[0], W[3], W[4]}, wc1 = d3{W[3], W[1], W[5]}, wc2 = d3{W[4], W[5], W[2]};
-                    const d3 y0 = cross3(c, wc0), y1 = cross3(c, wc1), y2 = cross3(c, wc2);
+                    // (roundings spelled out; the y as in assemble_rows)
+                    const d3 y0 = cross_rn(c, wc0), y2 = cross_rn(c, wc2);
+                    d3 y1 = cross_rn(c, wc1);
+                    y1.y = __fma_rn(-c.x, wc1.z, __dmul_rn(c.z, wc1.x));
                     // Z = C Y^T: column k of Z = c x (row k of Y)
-                    const d3 z0 = cross3(c, d3{y0.x, y1.x, y2.x});
-                    const d3 z1 = cross3(c, d3{y0.y, y1.y, y2.y});
-                    const d3 z2 = cross3(c, d3{y0.z, y1.z, y2.z});
+                    d3 z0 = cross_rn(c, d3{y0.x, y1.x, y2.x});
+                    d3 z1 = cross_rn(c, d3{y0.y, y1.y, y2.y});
+                    z0.y = __fma_rn(-c.x, y2.x, __dmul_rn(c.z, y0.x));
+                    z0.z = __fma_rn(-c.y, y0.x, __dmul_rn(c.x, y1.x));
+                    z1.z = __fma_rn(-c.y, y0.y, __dmul_rn(c.x, y1.y));
+                    const d3 z2 = cross_rn(c, d3{y0.z, y1.z, y2.z});
                     P[pk(0, 0)] += W[0]; P[pk(1, 0)] += W[3]; P[pk(1, 1)] += W[1];
                     P[pk(2, 0)] += W[4]; P[pk(2, 1)] += W[5]; P[pk(2, 2)] += W[2];
                     P[pk(3, 0)] += y0.x; P[pk(3, 1)] += y1.x; P[pk(3, 2)] += y2.x;
@@ -860,7 +946,7 @@ class SceneSolver {
             bool lin_bad = false;
             if (dense_mode) {
                 if constexpr (kLargeTeam) lin_bad = !dense_solve_warp();
-                else lin_bad = !direct_solve();
+                else lin_bad = Team::kind == 0 && in_smem ? !direct_solve<Team::kind == 0>() : !direct_solve<false>();
             }
             // mixed precision: FP32 PCG with FP64 refinement where PCG runs; an
             // inner breakdown or a refinement that stops converging falls back
@@ -901,7 +987,7 @@ class SceneSolver {
                         B.du[6 * gb + r] = (bn > 0 && attempt == 0) ? B.dsc[6 * gb + r] * B.du[6 * gb + r] : 0.0;
                 }
                 T.sync();
-                spmv_to_X(B.du, nullptr, 0.0);
+                spmv_to_X(B.du);
                 T.sync();
             }
             double s2[2] = {0, 0};
@@ -1016,18 +1102,17 @@ class SceneSolver {
             // retrieveNonSmoothForceInc (:254-280)
             for (int c = tid; c < nc; c += nt) {
                 const int gc = c0 + c;
-                const d3 w = rel_vel(gc, B.du);
-                st3(B.wd + 3 * gc, w);
-                double d0 = B.sf[3 * gc] - w.x, d1 = B.sf[3 * gc + 1] - w.y, d2 = B.sf[3 * gc + 2] - w.z;
-                d0 = B.knInv[gc] * d0;
-                const double t00 = B.ktInv[3 * gc], t01 = B.ktInv[3 * gc + 1], t11 = B.ktInv[3 * gc + 2];
-                const double e1 = t00 * d1 + t01 * d2, e2 = t01 * d1 + t11 * d2;
-                B.df[3 * gc] = d0;
-                B.df[3 * gc + 1] = e1;
-                B.df[3 * gc + 2] = e2;
-                B.dl[2 * gc] = -B.invC[2 * gc] * (-B.lam[2 * gc] * d0 + B.rl[2 * gc]);
-                B.dl[2 * gc + 1] = -B.invC[2 * gc + 1] *
-                                   (B.lam[2 * gc + 1] * (B.gr[2 * gc] * e1 + B.gr[2 * gc + 1] * e2) + B.rl[2 * gc + 1]);
+                double* const P = contact(gc);
+                const d3 w = rel_vel(gc, P, B.du);
+                fst3(P, F_wd, w);
+                const d3 d = sub3(fld3(P, F_sf), w);
+                const double d0 = P[32 * F_knInv] * d.x;
+                const d3 t = fld3(P, F_ktInv);
+                const double e1 = t.x * d.y + t.y * d.z, e2 = t.y * d.y + t.z * d.z;
+                fst3(P, F_df, d3{d0, e1, e2});
+                P[32 * F_dl] = -P[32 * F_invC] * (-P[32 * F_lam] * d0 + P[32 * F_rl]);
+                P[32 * (F_dl + 1)] = -P[32 * (F_invC + 1)] * (P[32 * (F_lam + 1)] * (P[32 * F_gr] * e1 + P[32 * (F_gr + 1)] * e2) +
+                                                        P[32 * (F_rl + 1)]);
             }
             T.sync();
             t1 = now();
@@ -1049,10 +1134,11 @@ class SceneSolver {
                 }
                 for (int c = tid; c < nc; c += nt) {
                     const int gc = c0 + c;
-                    st3(B.wd + 3 * gc, scl3(-1.0, rel_vel(gc, B.ru)));  // J du with du = -ru
-                    for (int r = 0; r < 3; ++r) B.df[3 * gc + r] = B.rf[3 * gc + r];
-                    B.dl[2 * gc] = B.rl[2 * gc];
-                    B.dl[2 * gc + 1] = B.rl[2 * gc + 1];
+                    double* const P = contact(gc);
+                    fst3(P, F_wd, scl3(-1.0, rel_vel(gc, P, B.ru)));  // J du with du = -ru
+                    fst3(P, F_df, fld3(P, F_rf));
+                    P[32 * F_dl] = P[32 * F_rl];
+                    P[32 * (F_dl + 1)] = P[32 * (F_rl + 1)];
                 }
                 T.sync();
                 step = line_search(sErr, sacErr, muc, C.gd_max, trials);
@@ -1166,14 +1252,16 @@ class SceneSolver {
         int* lvl_start;  // [levels + 1] first entry of each level in lvl_cols
         int* lvl_blk;    // [levels + 1] first block of each level
         int* lvl_len;    // [levels] longest update list of the level
-        int* meta;       // [0] levels, [1] blocks, [2] update-list entries
-        int* lbeg;       // [blocks + 1] start of each block's update list
-        unsigned short* ku;  // [blocks] (column << 8) | row of each block
-        double* Linv;    // [kSparseMax][kInvStride] packed inverse of each diagonal Cholesky factor
-        double* y;       // [kSparseMax][6] right-hand side, then L^-1 of it
-        double* x;       // [kSparseMax][6]
-        double* L;       // [cap][36] blocks
-        int cap;         // blocks
+        int* lvl_pat;    // [levels] most off-diagonal blocks of a column of the level
+        int* meta;       // [0] levels, [1] blocks, [2] update-list entries (0: no lists)
+        int4* desc;      // [blocks] first list entry; list length | column << 16 | row << 24;
+                         // first and one past the last contact (slot, or entry of inc_g)
+        double* y;       // [n + 1][6] right-hand side, then L^-1 of it, then the solution; node n is 0
+        double* L;       // [blocks + 1][36], each in the order of frag(); a diagonal block
+                         // becomes its Cholesky factor; the last is 0
+        const uint32_t* list;  // update lists, each padded to an even length
+        double* slot;    // [cap][36] room of the team's slot, for the blocks (when they
+        int cap;         // do not fit the shared memory) and then the lists
     };
     __device__ __forceinline__ Direct direct_ws() const {
         // thread-block teams use slot blockIdx.x of B.dense, warp teams slot
@@ -1184,11 +1272,11 @@ class SceneSolver {
         const long long stride = warp_slot ? B.dense_stride_warp : B.dense_stride;
         constexpr int M8 = kSparseMax + 8;
         Direct S;
-        double* d = first;
-        S.Linv = d; d += kInvStride * kSparseMax;
-        S.y = d; d += 6 * kSparseMax;
-        S.x = d; d += 6 * kSparseMax;
-        int* q = reinterpret_cast<int*>(d);
+        int4* d = reinterpret_cast<int4*>(first);
+        S.desc = d; d += kBlockCap + 2;
+        double* v = reinterpret_cast<double*>(d);
+        S.y = v; v += 6 * (kSparseMax + 2);
+        int* q = reinterpret_cast<int*>(v);
         S.colb = reinterpret_cast<uint32_t*>(q); q += kSparseMax * kSparseWords;
         S.rowb = reinterpret_cast<uint32_t*>(q); q += kSparseMax * kSparseWords;
         S.adj = reinterpret_cast<uint32_t*>(q); q += kSparseMax * kSparseWords;
@@ -1202,12 +1290,25 @@ class SceneSolver {
         S.lvl_start = q; q += M8;
         S.lvl_blk = q; q += M8;
         S.lvl_len = q; q += M8;
-        S.meta = q; q += 8;
-        S.lbeg = q; q += kBlockCap + 8;
-        S.ku = reinterpret_cast<unsigned short*>(q);
-        S.L = first + (kSparseHeaderBytes + 255) / 256 * 32 - 36LL * kSparseMax;
-        S.cap = (int)((stride - (S.L - first)) / 36);
+        S.lvl_pat = q; q += M8;
+        S.meta = q;
+        S.slot = first + (kSparseHeaderBytes + 255) / 256 * 32 - 36LL * (kSparseMax + 2);
+        S.cap = (int)((stride - (S.slot - first)) / 36) - 2;
+        S.L = S.slot;
+        if constexpr (Team::kind == 0) S.y = block_smem();
+        S.list = reinterpret_cast<const uint32_t*>(in_smem ? S.slot : S.slot + 36LL * (S.meta[1] + 2));
         return S;
+    }
+    // The thread block's dynamic shared memory (node vector, then blocks).
+    __device__ __forceinline__ static double* block_smem() {
+        extern __shared__ __align__(16) double s_direct[];
+        return s_direct;
+    }
+    // The blocks' address: shared memory when the factor fits there.
+    template <bool SM>
+    __device__ __forceinline__ static double* block_base(const Direct& S) {
+        if constexpr (SM) return block_smem() + kSmemVector;
+        else return S.L;
     }
     // rank of node u among the set bits of a column pattern (= its block slot)
     __device__ __forceinline__ static int bit_rank(const uint32_t* w, int u) {
@@ -1229,7 +1330,11 @@ class SceneSolver {
         const Direct S = direct_ws();
         constexpr int W = kSparseWords;
         const int n = n_active;
-        uint32_t* const adj = T.adjacency(S.adj);
+        uint32_t* adj = S.adj;
+        if constexpr (Team::kind == 0) {  // where the blocks will be
+            if (B.smem_blocks * 288 >= kSparseMax * kSparseWords * 4)
+                adj = reinterpret_cast<uint32_t*>(block_smem() + kSmemVector);
+        }
         for (int q = tid; q < n * W; q += nt) adj[q] = 0;
         T.sync();
         for (int l = tid; l < n_local; l += nt) {
@@ -1331,52 +1436,54 @@ class SceneSolver {
             S.lvl_start[l] = c;
             S.lvl_blk[l] = b;
             S.lvl_len[l] = 0;
+            S.lvl_pat[l] = 0;
         }
         if (tid == 0) S.meta[0] = nlev;
         T.sync();
         const int nblk = S.meta[1];
         if (nblk > S.cap) return false;
-        // (column, row) of every block
+        // (column, row) and list length of every block: block (u, k) takes L(u, d)
+        // L(k, d)^T for every d in the rows of both
         for (int q = tid; q < n * W; q += nt) {
             const int k = q / W, w = q - k * W;
             int b = S.base[k] + 1;
             for (int x = 0; x < w; ++x) b += __popc(S.colb[k * W + x]);
             uint32_t bits = S.colb[q];
+            if (w == 0) S.desc[S.base[k]].y = (k << 16) | (k << 24);
             while (bits) {
-                S.ku[b++] = (unsigned short)((k << 8) | ((w << 5) + __ffs(bits) - 1));
+                S.desc[b++].y = (k << 16) | (((w << 5) + __ffs(bits) - 1) << 24);
                 bits &= bits - 1;
             }
-            if (w == 0) S.ku[S.base[k]] = (unsigned short)((k << 8) | k);
         }
         T.sync();
-        // update lists: block (u, k) takes L(u, d) L(k, d)^T for every d in the
-        // rows of both
-        T.scan(nblk, 0,
-               [&](int i) {
-                   const int k = S.ku[i] >> 8, u = S.ku[i] & 255;
-                   int c = 0;
-                   for (int w = 0; w < W; ++w) c += __popc(S.rowb[k * W + w] & S.rowb[u * W + w]);
-                   if (c) atomicMax(&S.lvl_len[S.deg[k]], c);
-                   return c;
-               },
+        for (int i = tid; i < nblk; i += nt) {
+            const int y = S.desc[i].y, k = (y >> 16) & 255, u = (y >> 24) & 255;
+            int c = 0;
+            for (int w = 0; w < W; ++w) c += __popc(S.rowb[k * W + w] & S.rowb[u * W + w]);
+            if (c) atomicMax(&S.lvl_len[S.deg[k]], c);
+            if (k == u) atomicMax(&S.lvl_pat[S.deg[k]], S.height[k] - 1);
+            S.desc[i].y = y | c;
+        }
+        T.sync();
+        T.scan(nblk, 0, [&](int i) { return ((S.desc[i].y & 0xffff) + 1) & ~1; },
                [&](int i, int excl) {
-                   S.lbeg[i] = excl;
-                   if (i == nblk - 1) {
-                       const int k = S.ku[i] >> 8, u = S.ku[i] & 255;
-                       int c = 0;
-                       for (int w = 0; w < W; ++w) c += __popc(S.rowb[k * W + w] & S.rowb[u * W + w]);
-                       S.lbeg[nblk] = excl + c;
-                   }
+                   S.desc[i].x = excl;
+                   if (i == nblk - 1) S.meta[2] = excl + (((S.desc[i].y & 0xffff) + 1) & ~1);
                });
         T.sync();
-        const int total = S.lbeg[nblk];
-        const bool listed = total > 0 && (long long)total * 4 <= (long long)(S.cap - nblk) * 288;
-        if (tid == 0) S.meta[2] = listed ? total : 0;
-        if (listed) {
-            uint32_t* const list = reinterpret_cast<uint32_t*>(S.L + 36LL * nblk);
+        const int total = S.meta[2];
+        in_smem = Team::kind == 0 && nblk + 2 <= B.smem_blocks;
+        const int used = in_smem ? 0 : nblk + 2;
+        const bool listed = (long long)total * 4 <= (long long)(S.cap - used) * 288;
+        if (!listed) {
+            T.sync();  // everyone has read the total
+            if (tid == 0) S.meta[2] = 0;
+        } else {
+            uint32_t* const list = reinterpret_cast<uint32_t*>(S.slot + 36LL * used);
             for (int i = tid; i < nblk; i += nt) {
-                const int k = S.ku[i] >> 8, u = S.ku[i] & 255;
-                int o = S.lbeg[i];
+                const int4 d = S.desc[i];
+                const int k = (d.y >> 16) & 255, u = (d.y >> 24) & 255;
+                int o = d.x;
                 for (int w = 0; w < W; ++w) {
                     uint32_t bits = S.rowb[k * W + w] & S.rowb[u * W + w];
                     while (bits) {
@@ -1384,22 +1491,36 @@ class SceneSolver {
                         bits &= bits - 1;
                     }
                 }
+                if (d.y & 1) list[o] = zero_entry(S, k, u);
             }
         }
-        // the block each incidence adds to: L(u, k) of its two bodies' positions,
-        // kept by the body eliminated first (-1: the other body keeps it, or the
-        // other body is static); inc_o is the PCG's and free here
+        // the contacts of each off-diagonal block: of a body's incidences those
+        // whose other body is eliminated later, grouped by block, in incidence
+        // order (inc_o is the PCG's and holds the incidence's block meanwhile)
         for (int k = tid; k < n; k += nt) {
             const int gb = S.body[k];
             const int st0 = B.inc_start[gb], cnt = B.inc_cnt[gb];
+            const int b0k = S.base[k] + 1, b1k = S.base[k] + S.height[k];
+            S.desc[b0k - 1].z = st0;  // the diagonal block takes all of them
+            S.desc[b0k - 1].w = st0 + cnt;
+            for (int b = b0k; b < b1k; ++b) S.desc[b].z = 0;
             for (int q = 0; q < cnt; ++q) {
                 const int go = B.inc_o[st0 + q];
                 int blk = -1;
                 if (go >= 0 && go != gb && B.local[go]) {
                     const int u = S.ipos[B.didx[go]];
-                    if (u > k) blk = S.base[k] + 1 + bit_rank(S.colb + k * W, u);
+                    if (u > k) {
+                        blk = b0k + bit_rank(S.colb + k * W, u);
+                        S.desc[blk].z += 1;
+                    }
                 }
                 B.inc_o[st0 + q] = blk;
+            }
+            int o = st0;  // ends of the blocks' ranges, then each range filled from its end
+            for (int b = b0k; b < b1k; ++b) S.desc[b].z = S.desc[b].w = o += S.desc[b].z;
+            for (int q = cnt - 1; q >= 0; --q) {
+                const int blk = B.inc_o[st0 + q];
+                if (blk >= 0) B.inc_g[S.desc[blk].z -= 1] = st0 + q;
             }
         }
         T.sync();
@@ -1412,6 +1533,11 @@ class SceneSolver {
         const uint32_t* cd = S.colb + d * kSparseWords;
         const uint32_t a = (uint32_t)(S.base[d] + 1 + bit_rank(cd, u));
         return (a << 16) | (u == k ? (uint32_t)d : (uint32_t)(S.base[d] + 1 + bit_rank(cd, k)));
+    }
+    // The entry that pads a list to an even length: the zero block (and node).
+    __device__ __forceinline__ uint32_t zero_entry(const Direct& S, int k, int u) const {
+        const uint32_t z = (uint32_t)S.meta[1];
+        return (z << 16) | (u == k ? (uint32_t)n_active : z);
     }
 
     // Symbolic factorisation on the large-scene teams (up to kSparseMaxLarge
@@ -1436,6 +1562,11 @@ class SceneSolver {
         z ^= z >> 31;
         return ((unsigned long long)deg << 32) | ((z >> 48) << 16) | (unsigned long long)i;
     }
+    // Sequential work of a column with m off-diagonal blocks and a row list of
+    // `len` entries: row updates per lane, plus its level's fixed cost.
+    __device__ __forceinline__ static int column_work(int m, int len) {
+        return kLevelCost + ((6 * (m + 1) + 31) >> 5) * (1 + len);
+    }
     __device__ bool sparse_symbolic_large() {
         Sparse S = sparse_ws();
         const int n = n_active, nw = (n + 31) >> 5;
@@ -1450,6 +1581,7 @@ class SceneSolver {
             S.height[q] = 0;
             S.lvl_start[q] = 0;
             S.lvl_work[q] = 0;
+            S.cstart[q] = 0;  // columns eliminated so far whose pattern holds the node
         }
         T.sync();
         for (int l = tid; l < n_local; l += nt) {  // node rows, each built by its owner
@@ -1473,6 +1605,7 @@ class SceneSolver {
         }
         T.sync();
         int done = 0;
+        double fill = 0;
         for (int round = 0; round < kMmdMaxRounds; ++round) {
             double m[1] = {-1e300};  // minimum degree over the remaining nodes
             for (int i = tid; i < n; i += nt)
@@ -1512,10 +1645,22 @@ class SceneSolver {
                        }
                    });
             {
-                double c[1] = {0.0};  // nodes eliminated this round
-                for (int i = tid; i < n; i += nt) c[0] += S.sel[i];
+                // Nodes eliminated this round, and what their columns add to the
+                // factor's blocks and to its depth (their patterns, heights and
+                // row lists are final).  Both only grow, so a factor that will
+                // not fit or will be too deep is left as soon as it is: the last
+                // rounds, one node of a dense separator each, cost the most.
+                double c[2] = {0.0, 0.0};
+                for (int i = tid; i < n; i += nt) {
+                    if (!S.sel[i]) continue;
+                    c[0] += 1;
+                    c[1] += S.deg[i];
+                    atomicMax(&S.lvl_work[S.height[i]], column_work(S.deg[i], S.cstart[i]));
+                }
                 T.sum(c);
                 done += (int)c[0];
+                fill += c[1];
+                if (fill > S.cap || fill > kRowCapLarge) return false;
             }
             for (int u = tid; u < n; u += nt) {  // remaining neighbours merge the eliminated patterns
                 if (S.ipos[u] >= 0) continue;
@@ -1529,6 +1674,7 @@ class SceneSolver {
                         bits &= bits - 1;
                         if (!S.sel[v]) continue;
                         touched = true;
+                        S.cstart[u] += 1;
                         h = max(h, S.height[v] + 1);
                         const uint32_t* av = S.adj + v * W;
                         for (int x = 0; x < nw; ++x) au[x] |= av[x];
@@ -1543,7 +1689,10 @@ class SceneSolver {
                     S.height[u] = h;
                 }
             }
-            T.sync();
+            double depth[1] = {0.0};
+            for (int l = tid; l < n; l += nt) depth[0] += S.lvl_work[l];
+            T.sum(depth);
+            if (depth[0] > kDirectDepthMax) return false;
         }
         if (done != n) return false;  // round limit
         // block offsets in elimination order
@@ -1621,8 +1770,7 @@ class SceneSolver {
             S.lvl_nodes[atomicAdd(&S.deg[S.height[v]], 1)] = v;
             int m = 0;
             for (int w = 0; w < nw; ++w) m += __popc(S.adj[v * W + w]);
-            const int wk = kLevelCost + ((6 * (m + 1) + 31) >> 5) * (1 + S.rowptr[v + 1] - S.rowptr[v]);
-            atomicMax(&S.lvl_work[S.height[v]], wk);
+            atomicMax(&S.lvl_work[S.height[v]], column_work(m, S.rowptr[v + 1] - S.rowptr[v]));
         }
         T.sync();
         double depth[1] = {0.0};
@@ -1657,9 +1805,9 @@ class SceneSolver {
             double* blk = col + 36 * bit_rank(ai, j);
             // block (rows o, cols b) = -[[W, C_b W]^T-form]: the transpose of
             // A_bo = -[[W, W C_o^T], [C_b W, C_b W C_o^T]]
-            const double* W = B.W + 6 * gc;
-            const d3 cb = ld3(B.arm + 6 * gc + 3 * side);
-            const d3 co = ld3(B.arm + 6 * gc + 3 * (1 - side));
+            double W[12];
+            ldg12(st0 + k, W);
+            const d3 cb = ld3(W + 6), co = ld3(W + 9);
             const d3 wr[3] = {d3{W[0], W[3], W[4]}, d3{W[3], W[1], W[5]}, d3{W[4], W[5], W[2]}};
             const d3 y0 = cross3(cb, wr[0]), y1 = cross3(cb, wr[1]), y2 = cross3(cb, wr[2]);
             const d3 yr[3] = {d3{y0.x, y1.x, y2.x}, d3{y0.y, y1.y, y2.y}, d3{y0.z, y1.z, y2.z}};
@@ -1721,282 +1869,362 @@ class SceneSolver {
             x[i] = t * Li[i];
         }
     }
-    // Inverse of the lower Cholesky factor of a 6x6 SPD block (row-major, lower
-    // triangle read), packed by rows; false if not SPD.  One reciprocal square
-    // root per column is the whole chain: the diagonal of the factor itself is
-    // never needed.
-    __device__ __forceinline__ static bool chol6_inverse(const double* A, double* Li) {
-        double L[15], inv[6];  // strictly lower factor, packed by rows
-#pragma unroll
-        for (int j = 0; j < 6; ++j) {
-            double d = A[7 * j];
-#pragma unroll
-            for (int k = 0; k < j; ++k) d -= L[j * (j - 1) / 2 + k] * L[j * (j - 1) / 2 + k];
-            if (!(d > 0.0)) return false;
-            inv[j] = rsqrt(d);
-#pragma unroll
-            for (int i = j + 1; i < 6; ++i) {
-                double t = A[6 * i + j];
-#pragma unroll
-                for (int k = 0; k < j; ++k) t -= L[i * (i - 1) / 2 + k] * L[j * (j - 1) / 2 + k];
-                L[i * (i - 1) / 2 + j] = t * inv[j];
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 6; ++i) {
-#pragma unroll
-            for (int j = 0; j < i; ++j) {
-                double t = 0.0;
-#pragma unroll
-                for (int k = j; k < i; ++k) t += L[i * (i - 1) / 2 + k] * Li[k * (k + 1) / 2 + j];
-                Li[i * (i + 1) / 2 + j] = -t * inv[i];
-            }
-            Li[i * (i + 1) / 2 + i] = inv[i];
-        }
-        return true;
+    // Position of element (r, c) of a 6x6 block in memory: columns 0-3 by rows,
+    // then columns 4-5 by rows.  Lanes 0-23 of a warp read the first 24 doubles
+    // as the k = 0..3 operand of an m8n8k4 product in one run, the last 12 give
+    // half of a second operand, and a row is three aligned pairs.
+    __device__ __forceinline__ static constexpr int frag(int r, int c) { return c < 4 ? 4 * r + c : 24 + 2 * r + c - 4; }
+    __device__ __forceinline__ static void st_row(double* p, int r, const double* v) {
+        *reinterpret_cast<double2*>(p + 4 * r) = make_double2(v[0], v[1]);
+        *reinterpret_cast<double2*>(p + 4 * r + 2) = make_double2(v[2], v[3]);
+        *reinterpret_cast<double2*>(p + 24 + 2 * r) = make_double2(v[4], v[5]);
     }
-    __device__ __forceinline__ static void ld6(const double* p, double* v) {  // 16-byte aligned
-        const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1],
-                      c = reinterpret_cast<const double2*>(p)[2];
+    // (c0, c1) += A B for the warp's 8x4 A (a = A[lane / 4][lane % 4]), 4x8 B (b =
+    // B[lane % 4][lane / 4]); the lane holds C[lane / 4][2 (lane % 4) + {0, 1}]
+    __device__ __forceinline__ static void mma884(double& c0, double& c1, double a, double b) {
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                     : "+d"(c0), "+d"(c1)
+                     : "d"(a), "d"(b));
+    }
+
+    __device__ __forceinline__ static void ld_row(const double* p, int r, double* v) {
+        const double2 a = *reinterpret_cast<const double2*>(p + 4 * r), b = *reinterpret_cast<const double2*>(p + 4 * r + 2),
+                      c = *reinterpret_cast<const double2*>(p + 24 + 2 * r);
         v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y;
     }
-    __device__ __forceinline__ static void st6(double* p, const double* v) {
-        reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
-        reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
-        reinterpret_cast<double2*>(p)[2] = make_double2(v[4], v[5]);
+    // In place: the strictly lower part of a 6x6 SPD block's Cholesky factor and
+    // the reciprocals of its diagonal (all that the substitutions read), and
+    // y = L^-1 y; false if not SPD.
+    __device__ __forceinline__ static bool chol6_block(double* A, double* y) {
+        double L[6][6], inv[6];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            double d = A[frag(j, j)];
+#pragma unroll
+            for (int k = 0; k < j; ++k) d -= L[j][k] * L[j][k];
+            if (!(d > 0.0)) return false;
+            inv[j] = 1.0 / sqrt(d);
+#pragma unroll
+            for (int i = j + 1; i < 6; ++i) {
+                double t = A[frag(i, j)];
+#pragma unroll
+                for (int k = 0; k < j; ++k) t -= L[i][k] * L[j][k];
+                L[i][j] = t * inv[j];
+            }
+        }
+        double b[6];
+        ld6(y, b);
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            A[frag(i, i)] = inv[i];
+            double t = b[i];
+#pragma unroll
+            for (int k = 0; k < i; ++k) {
+                A[frag(i, k)] = L[i][k];
+                t -= L[i][k] * b[k];
+            }
+            b[i] = t * inv[i];
+        }
+        st6(y, b);
+        return true;
     }
 
     // The Newton matrix and right-hand side of the block and warp teams' factor
-    // (linsysAddition's four blocks, :232-247), one thread per block row: row r of
-    // block (u, k) = T_u W T_k^T summed over the contacts of the two bodies in
-    // incidence order, T_j = s_j [I; C_j] with C_j = [c_j]x, i.e. from the 3x3
-    // blocks [W, W C_k^T; C_u W, C_u W C_k^T] with the sign of s_u s_k; a diagonal
-    // row takes every contact of the body, M / cm + eps I, and component r of
-    // rhs = sum T_j K^-1 sf - ru; rows of blocks that only fill in are zero.
+    // (linsysAddition's four blocks, :232-247), one thread per pair of rows i, 3 +
+    // i of a block: block (u, k) = T_u W T_k^T summed over the contacts of the two
+    // bodies in incidence order, T_j = s_j [I; C_j] with C_j = [c_j]x, with the
+    // sign of s_u s_k, i.e. [W, (C_k W)^T; C_u W, C_u (C_k W)^T]; a diagonal block
+    // starts from M / cm + eps I, takes every contact of the body, and its threads
+    // also sum rhs = sum T_j K^-1 sf - ru; blocks that only fill in are zero.  The
+    // three threads of a block run the same instructions (component i of a cross
+    // product by selecting its two factors).  Roundings are spelled out (which of
+    // a cross product's two terms is fused), so that a change elsewhere in the
+    // kernel cannot move the results of scenes that amplify the last bit.
+    template <bool SM>
     __device__ void assemble_rows(double eps) const {
         const Direct S = direct_ws();
-        const int rows = 6 * S.meta[1];
-        for (int t = tid; t < rows; t += nt) {
-            const int i = t / 6, r = t - 6 * i;
-            const int k = S.ku[i] >> 8, u = S.ku[i] & 255;
-            const int gb = S.body[k], st0 = B.inc_start[gb], cnt = B.inc_cnt[gb];
-            const bool diag = k == u;
-            double a[6] = {0, 0, 0, 0, 0, 0}, b = 0;
-            const int q3 = r < 3 ? r : r - 3;
-            for (int q = 0; q < cnt; ++q) {
-                if (!diag && B.inc_o[st0 + q] != i) continue;
-                const int e = B.inc[st0 + q], gc = e >> 1, side = e & 1;
-                const double* W = B.W + 6 * gc;
-                const d3 w0 = d3{W[0], W[3], W[4]}, w1 = d3{W[3], W[1], W[5]}, w2 = d3{W[4], W[5], W[2]};
-                const d3 ck = ld3(B.arm + 6 * gc + 3 * side);
-                const d3 cu = diag ? ck : ld3(B.arm + 6 * gc + 3 * (1 - side));
-                // row q3 of W, or of C_u W: (c x)_ab row q3 times W
-                d3 v;
-                if (r < 3) v = q3 == 0 ? w0 : (q3 == 1 ? w1 : w2);
-                else if (q3 == 0) v = sub3(scl3(cu.y, w2), scl3(cu.z, w1));
-                else if (q3 == 1) v = sub3(scl3(cu.z, w0), scl3(cu.x, w2));
-                else v = sub3(scl3(cu.x, w1), scl3(cu.y, w0));
-                const d3 z = cross3(ck, v);  // the row times C_k^T
+        double* const L = block_base<SM>(S);
+        const int nblk = S.meta[1], items = 3 * nblk;
+        for (int t = tid; t < items; t += nt) {
+            const int b = t / 3, i = t - 3 * b;
+            const int4 de = S.desc[b];
+            const int k = (de.y >> 16) & 255, u = (de.y >> 24) & 255, gb = S.body[k];
+            const bool diag = k == u, is0 = i == 0, is1 = i == 1;
+            auto pick = [&](double x, double y, double z) { return is0 ? x : (is1 ? y : z); };  // component i
+            auto cross_i = [&](double cp, double cq, d3 v) {  // component i of c x v, c_(i+1), c_(i+2) given
+                return __fma_rn(cp, pick(v.z, v.x, v.y), -__dmul_rn(cq, pick(v.y, v.z, v.x)));
+            };
+            double lo[6] = {0, 0, 0, 0, 0, 0}, hi[6] = {0, 0, 0, 0, 0, 0}, fl = 0, fh = 0;
+            if (diag) {
+                const double m = B.mass[gb] / cm + eps;
+                const double* I = B.inertia + 6 * gb;
+                const double xx = I[0] / cm + eps, yy = I[1] / cm + eps, zz = I[2] / cm + eps;
+                const double xy = I[3] / cm, xz = I[4] / cm, yz = I[5] / cm;
+                lo[0] = pick(m, 0.0, 0.0); lo[1] = pick(0.0, m, 0.0); lo[2] = pick(0.0, 0.0, m);
+                hi[3] = pick(xx, xy, xz); hi[4] = pick(xy, yy, yz); hi[5] = pick(xz, yz, zz);
+            }
+            for (int q = de.z; q < de.w; ++q) {
+                const int slot = diag ? q : B.inc_g[q];
+                double g[12];
+                ldg12(slot, g);
+                const d3 ck = ld3(g + 6), cu = diag ? ck : ld3(g + 9);
+                const d3 w0 = d3{g[0], g[3], g[4]}, w1 = d3{g[3], g[1], g[5]}, w2 = d3{g[4], g[5], g[2]};
+                const d3 y0 = cross_rn(ck, w0), y2 = cross_rn(ck, w2);  // columns of C_k W
+                d3 y1 = cross_rn(ck, w1);
+                y1.y = __fma_rn(-ck.x, w1.z, __dmul_rn(ck.z, w1.x));
+                const double s = diag ? 1.0 : -1.0;
+                lo[0] += s * pick(w0.x, w1.x, w2.x); lo[1] += s * pick(w0.y, w1.y, w2.y); lo[2] += s * pick(w0.z, w1.z, w2.z);
+                lo[3] += s * pick(y0.x, y1.x, y2.x); lo[4] += s * pick(y0.y, y1.y, y2.y); lo[5] += s * pick(y0.z, y1.z, y2.z);
+                const double cp = pick(cu.y, cu.z, cu.x), cq = pick(cu.z, cu.x, cu.y);
+                hi[0] += s * cross_i(cp, cq, w0);
+                hi[1] += s * (is1 ? __fma_rn(-cq, w1.z, __dmul_rn(cp, w1.x)) : cross_i(cp, cq, w1));
+                hi[2] += s * cross_i(cp, cq, w2);
+                hi[3] += s * cross_i(cp, cq, d3{y0.x, y1.x, y2.x});
+                hi[4] += s * cross_i(cp, cq, d3{y0.y, y1.y, y2.y});
+                hi[5] += s * cross_i(cp, cq, d3{y0.z, y1.z, y2.z});
                 if (diag) {
-                    a[0] += v.x; a[1] += v.y; a[2] += v.z; a[3] += z.x; a[4] += z.y; a[5] += z.z;
-                    const d3 x = ld3(B.Xi + 3LL * (st0 + q));
-                    const d3 h = r < 3 ? x : cross3(ck, x);
-                    b += q3 == 0 ? h.x : (q3 == 1 ? h.y : h.z);
-                } else {
-                    a[0] -= v.x; a[1] -= v.y; a[2] -= v.z; a[3] -= z.x; a[4] -= z.y; a[5] -= z.z;
+                    const d3 x = fld3(incidence(slot), I_X);
+                    fl += pick(x.x, x.y, x.z);
+                    fh += cross_i(cp, cq, x);
                 }
             }
             if (diag) {
-                if (r < 3) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c)
-                        if (c == r) a[c] += B.mass[gb] / cm + eps;
-                } else {
-                    const double* I = B.inertia + 6 * gb;
-                    const double ix = q3 == 0 ? I[0] : (q3 == 1 ? I[3] : I[4]);
-                    const double iy = q3 == 0 ? I[3] : (q3 == 1 ? I[1] : I[5]);
-                    const double iz = q3 == 0 ? I[4] : (q3 == 1 ? I[5] : I[2]);
-                    a[3] += ix / cm + (q3 == 0 ? eps : 0.0);
-                    a[4] += iy / cm + (q3 == 1 ? eps : 0.0);
-                    a[5] += iz / cm + (q3 == 2 ? eps : 0.0);
-                }
-                S.y[6 * k + r] = b - B.ru[6 * gb + r];
+                S.y[6 * k + i] = fl - B.ru[6 * gb + i];
+                S.y[6 * k + 3 + i] = fh - B.ru[6 * gb + 3 + i];
             }
-            st6(S.L + 36LL * i + 6 * r, a);
+            st_row(L + 36 * b, i, lo);
+            st_row(L + 36 * b, 3 + i, hi);
+        }
+        for (int t = tid; t < 36; t += nt) {
+            L[36 * nblk + t] = 0.0;
+            if (t < 6) S.y[6 * n_active + t] = 0.0;
         }
     }
 
-    // One row's update by column d: acc -= x L^T with x = row r of L(u, d), L =
-    // L(k, d) (both 6x6); a diagonal row also takes its share of the forward
-    // substitution, x . y_d.
-    __device__ __forceinline__ static void row_update(const Direct& S, uint32_t e, bool diag, int r, double* acc,
-                                                      double& yr) {
-        const double* A = S.L + 36LL * (e >> 16);
-        const double* Bm = diag ? A : S.L + 36LL * (e & 0xffffu);
-        double x[6];
-        ld6(A + 6 * r, x);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            double b[6];
-            ld6(Bm + 6 * c, b);
-            double t = x[0] * b[0];
-#pragma unroll
-            for (int q = 1; q < 6; ++q) t += x[q] * b[q];
-            acc[c] -= t;
+    // Entry `r` of block (u, k)'s update list without the list: the r-th column
+    // in the rows of both
+    __device__ __forceinline__ uint32_t find_entry(const Direct& S, int k, int u, int r) const {
+        for (int w = 0; w < kSparseWords; ++w) {
+            uint32_t x = S.rowb[k * kSparseWords + w] & S.rowb[u * kSparseWords + w];
+            const int c = __popc(x);
+            if (r < c) {
+                for (; r > 0; --r) x &= x - 1;
+                return update_entry(S, k, u, (w << 5) + __ffs(x) - 1);
+            }
+            r -= c;
         }
-        if (diag) {
-            double b[6];
-            ld6(S.y + 6 * (e & 0xffffu), b);
-            double t = x[0] * b[0];
+        return zero_entry(S, k, u);
+    }
+    // Block i = (u, k) -= the products of its update list, by one warp: two
+    // entries per round, the first four columns of each (heads) as one product
+    // and the last two of both in a third.  Rows 6 and 7 of the operands hold
+    // what lies there: they only reach rows and columns of the product that are
+    // not used, but for a diagonal block, which multiplies L(k, d) by its own
+    // transpose with y_d as row 6 of the second factor, so that column 6 of the
+    // product is the forward substitution's part.  One entry is 6 cycles of the
+    // load-store unit; a thread per block row, loading its factor's 36 values
+    // again for every row, took 29.
+    template <bool SM>
+    __device__ __forceinline__ void update_block(const Direct& S, double* L, int i, int4 de, bool listed,
+                                                 int lane) const {
+        const int row = lane >> 2, kk = lane & 3, n = de.y & 0xffff;
+        const int k = (de.y >> 16) & 255, u = (de.y >> 24) & 255;
+        const bool diag = k == u, ycol = diag && row == 6;
+        const int tail = 24 + 2 * row + (kk & 1);
+        const uint2* const list = reinterpret_cast<const uint2*>(S.list + de.x);
+        double s0 = 0, s1 = 0, t0 = 0, t1 = 0;
+        uint2 e = make_uint2(0, 0);
+        if (listed) e = list[0];
+        for (int q = 0; q < n; q += 2) {
+            uint2 now = e;
+            if (listed) {
+                if (q + 2 < n) e = list[(q >> 1) + 1];
+            } else {
+                now = make_uint2(find_entry(S, k, u, q), find_entry(S, k, u, q + 1));
+            }
+            const double* const A0 = L + 36 * (now.x >> 16);
+            const double* const A1 = L + 36 * (now.y >> 16);
+            const double a0 = A0[lane], a1 = A1[lane], at = (kk < 2 ? A0 : A1)[tail];
+            double b0, b1, bt;
+            if (diag) {
+                b0 = a0, b1 = a1, bt = at;
+                if (ycol) {
+                    const double *y0 = S.y + 6 * (now.x & 0xffffu), *y1 = S.y + 6 * (now.y & 0xffffu);
+                    b0 = y0[kk];
+                    b1 = y1[kk];
+                    bt = (kk < 2 ? y0 : y1)[4 + (kk & 1)];
+                }
+            } else {
+                const double* const B0 = L + 36 * (now.x & 0xffffu);
+                const double* const B1 = L + 36 * (now.y & 0xffffu);
+                b0 = B0[lane];
+                b1 = B1[lane];
+                bt = (kk < 2 ? B0 : B1)[tail];
+            }
+            mma884(s0, s1, a0, b0);
+            mma884(t0, t1, a1, b1);
+            mma884(s0, s1, at, bt);
+        }
+        s0 += t0;
+        s1 += t1;
+        if (row < 6) {
+            if (kk < 3) {
+                double2* c = reinterpret_cast<double2*>(L + 36 * i + (kk < 2 ? 4 * row + 2 * kk : 24 + 2 * row));
+                const double2 v = *c;
+                *c = make_double2(v.x - s0, v.y - s1);
+            } else if (diag) {
+                S.y[6 * k + row] -= s0;  // column 6
+            }
+        }
+    }
+
+    // The same for a level of short lists (at most kShortList entries): a thread
+    // per block row, entry by entry.
+    __device__ __forceinline__ void update_rows(const Direct& S, double* L, int i0, int i1, bool listed) const {
+        for (int t = tid; t < 6 * (i1 - i0); t += nt) {
+            const int i = i0 + t / 6, r = t - 6 * (i - i0);
+            const int4 de = S.desc[i];
+            const int n = de.y & 0xffff;
+            if (n == 0) continue;
+            const int k = (de.y >> 16) & 255, u = (de.y >> 24) & 255;
+            const bool diag = k == u;
+            double acc[6], yr = 0;
+            ld_row(L + 36 * i, r, acc);
+            if (diag) yr = S.y[6 * k + r];
+            for (int q = 0; q < n; ++q) {
+                const uint32_t e = listed ? S.list[de.x + q] : find_entry(S, k, u, q);
+                const double* const A = L + 36 * (e >> 16);
+                const double* const Bm = diag ? A : L + 36 * (e & 0xffffu);
+                double x[6], b[6];
+                ld_row(A, r, x);
 #pragma unroll
-            for (int q = 1; q < 6; ++q) t += x[q] * b[q];
-            yr -= t;
+                for (int c = 0; c < 6; ++c) {
+                    ld_row(Bm, c, b);
+                    double s = 0.0;
+#pragma unroll
+                    for (int p = 0; p < 6; ++p) s += x[p] * b[p];
+                    acc[c] -= s;
+                }
+                if (diag) {
+                    ld6(S.y + 6 * (e & 0xffffu), b);
+                    double s = 0.0;
+#pragma unroll
+                    for (int p = 0; p < 6; ++p) s += x[p] * b[p];
+                    yr -= s;
+                }
+            }
+            st_row(L + 36 * i, r, acc);
+            if (diag) S.y[6 * k + r] = yr;
         }
     }
 
     // Block Cholesky factorisation and both substitutions of the Newton system
     // (block and warp teams; left-looking), one elimination-tree level at a time,
-    // the forward substitution riding along as one more component of each
-    // diagonal row.  Per level: (1) every row of the level's blocks takes its
-    // updates (the block's list of earlier blocks), a level with few rows giving
-    // each row 2 to 32 adjacent lanes that split the list and combine by an xor
-    // butterfly; (2) a thread per column inverts the Cholesky factor of its
-    // diagonal block and finishes its part of the forward substitution; (3) the
-    // other rows are scaled, A(u, k) L_kk^-T.  The backward substitution gives a
-    // column 8, 16 or 32 lanes (component x blocks) and no barrier but the
-    // level's.  Every scene of a batch spends most of its time here, bound by the
-    // chain of dependent loads of each level.  Looking up patterns bit by bit
-    // for every block product, one lane factoring and writing back a diagonal
-    // block, whole subtrees in sequence per warp and a separate forward sweep
-    // took 1,340 us per Newton iteration on a crate of 144 cubes and 49 us on a
-    // 10-box stack; this takes 750 and 32 us.  Stands in for the direct branch's
-    // SimplicialLDLT (:385-394).  Writes du; false on a non-SPD pivot, which only
-    // marks the scene: later columns then compute garbage in bounded loops.
+    // the forward substitution riding along as one more column of each diagonal
+    // block.  Per level: (1) the blocks take their updates, a warp per block or,
+    // where the lists are short, a thread per row; (2) a thread per column
+    // factors its diagonal block and finishes its part of the forward
+    // substitution; (3) a thread per row scales the other blocks, A(u, k) L_kk^-T.
+    // The backward substitution gives a column 8, 16 or 32 lanes (component x
+    // blocks) and no barrier but the level's.  Levels of short lists and patterns
+    // (stacks, columns, loose piles) sum entry by entry in elimination order.
+    // Long lists run on the FP64 matrix instruction: it has the rate of the FP64
+    // pipe, but feeds 256 multiply-adds from two loads per lane.  Stands in for
+    // the direct branch's SimplicialLDLT (:385-394).  Writes du; false on a
+    // non-SPD pivot, which only marks the scene: later columns then compute
+    // garbage in bounded loops.
+    template <bool SM>
     __device__ bool direct_solve() {
         const Direct S = direct_ws();
-        const int nlev = S.meta[0], nblk = S.meta[1];
+        double* const L = block_base<SM>(S);
+        const int nlev = S.meta[0];
         const bool listed = S.meta[2] > 0;
-        const uint32_t* const list = reinterpret_cast<const uint32_t*>(S.L + 36LL * nblk);
+        const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
         bool bad = false;
+        int q1 = 0, i1 = 0;
         for (int l = 0; l < nlev; ++l) {
-            const int q0 = S.lvl_start[l], q1 = S.lvl_start[l + 1];
-            const int i0 = S.lvl_blk[l], rows = 6 * (S.lvl_blk[l + 1] - i0), len = S.lvl_len[l];
+            const int q0 = q1, i0 = i1;
+            q1 = S.lvl_start[l + 1];
+            i1 = S.lvl_blk[l + 1];
+            const int len = S.lvl_len[l];
             if (len > 0) {
-                int split = 1;
-                if (listed)
-                    while (split < 32 && split < len && rows * split * 2 <= nt) split *= 2;
-                for (int t0 = 0; t0 < rows; t0 += nt) {  // split > 1: one round
-                    const int t = t0 + tid / split, j = tid & (split - 1);
-                    const bool on = t < rows;
-                    const int i = i0 + (on ? t : 0) / 6, r = on ? t - 6 * (i - i0) : 0;
-                    const int k = S.ku[i] >> 8, u = S.ku[i] & 255;
-                    const bool diag = k == u;
-                    double acc[6] = {0, 0, 0, 0, 0, 0}, yr = 0;
-                    if (on && j == 0) {
-                        ld6(S.L + 36LL * i + 6 * r, acc);
-                        if (diag) yr = S.y[6 * k + r];
-                    }
-                    if (on && listed) {
-                        for (int q = S.lbeg[i] + j; q < S.lbeg[i + 1]; q += split)
-                            row_update(S, list[q], diag, r, acc, yr);
-                    } else if (on) {
-                        for (int w = 0; w <= (k >> 5); ++w) {
-                            uint32_t bits = S.rowb[k * kSparseWords + w] & S.rowb[u * kSparseWords + w];
-                            while (bits) {
-                                row_update(S, update_entry(S, k, u, (w << 5) + __ffs(bits) - 1), diag, r, acc, yr);
-                                bits &= bits - 1;
-                            }
-                        }
-                    }
-                    for (int o = 1; o < split; o <<= 1) {
-#pragma unroll
-                        for (int c = 0; c < 6; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-                        yr += __shfl_xor_sync(0xffffffffu, yr, o);
-                    }
-                    if (on && j == 0) {
-                        st6(S.L + 36LL * i + 6 * r, acc);
-                        if (diag) S.y[6 * k + r] = yr;
+                if (len <= kShortList) {
+                    update_rows(S, L, i0, i1, listed);
+                } else {
+                    for (int i = i0 + warp; i < i1; i += nwarp) {
+                        const int4 de = S.desc[i];
+                        if ((de.y & 0xffff) != 0) update_block<SM>(S, L, i, de, listed, lane);
                     }
                 }
                 T.sync();
             }
             for (int q = q0 + tid; q < q1; q += nt) {
                 const int k = S.lvl_cols[q];
-                double Li[21], b[6];
-                if (!chol6_inverse(S.L + 36LL * S.base[k], Li)) {
-                    bad = true;
-                    continue;
-                }
-                ld6(S.y + 6 * k, b);
-                double* out = S.Linv + kInvStride * k;
-#pragma unroll
-                for (int c = 0; c < 21; ++c) out[c] = Li[c];
-                double y[6];
-#pragma unroll
-                for (int r = 0; r < 6; ++r) {
-                    double t = 0.0;
-#pragma unroll
-                    for (int c = 0; c <= r; ++c) t += Li[r * (r + 1) / 2 + c] * b[c];
-                    y[r] = t;
-                }
-                st6(S.y + 6 * k, y);
+                if (!chol6_block(L + 36 * S.base[k], S.y + 6 * k)) bad = true;
             }
             T.sync();
-            if (rows == 6 * (q1 - q0)) continue;  // no off-diagonal block in this level
-            for (int t = tid; t < rows; t += nt) {
+            if (i1 - i0 == q1 - q0) continue;  // no off-diagonal block in this level
+            for (int t = tid; t < 6 * (i1 - i0); t += nt) {
                 const int i = i0 + t / 6, r = t - 6 * (i - i0);
-                const int k = S.ku[i] >> 8;
-                if ((S.ku[i] & 255) == k) continue;
-                double* row = S.L + 36LL * i + 6 * r;
-                const double* Li = S.Linv + kInvStride * k;
-                double a[6], o[6];
-                ld6(row, a);
+                const int y = S.desc[i].y, k = (y >> 16) & 255;
+                if (((y >> 24) & 255) == k) continue;
+                const double* const D = L + 36 * S.base[k];
+                double a[6];
+                ld_row(L + 36 * i, r, a);
 #pragma unroll
                 for (int c = 0; c < 6; ++c) {
-                    double s = 0.0;
+                    double s = a[c];
 #pragma unroll
-                    for (int q = 0; q <= c; ++q) s += a[q] * Li[c * (c + 1) / 2 + q];
-                    o[c] = s;
+                    for (int q = 0; q < c; ++q) s -= D[frag(c, q)] * a[q];
+                    a[c] = s * D[frag(c, c)];
                 }
-                st6(row, o);
+                st_row(L + 36 * i, r, a);
             }
             T.sync();
         }
         if (T.any(bad)) return false;
-        const int c = min(tid & 7, 5), cc = tid & 7;
+        const int c8 = tid & 7, c = min(c8, 5);
+        const int e0 = c < 4 ? c : 20 + c, es = c < 4 ? 4 : 2;  // column c of a block: e0 + r es
+        int p1 = S.lvl_start[nlev];
         for (int l = nlev - 1; l >= 0; --l) {
-            const int q0 = S.lvl_start[l], ncol = S.lvl_start[l + 1] - q0;
-            int sub = 1;  // groups of 8 lanes per column
-            while (sub < 4 && ncol * 16 * sub <= nt) sub *= 2;
-            const int ng = nt / (8 * sub), grp = tid / (8 * sub), j = (tid >> 3) & (sub - 1);
+            const int p0 = S.lvl_start[l], ncol = p1 - p0;
+            p1 = p0;
+            // 1, 2 or 4 groups of 8 lanes per column
+            const int lg = S.lvl_pat[l] <= kShortList ? 0 : (ncol * 32 <= nt ? 2 : (ncol * 16 <= nt ? 1 : 0));
+            const int sub = 1 << lg;
+            const int ng = nt >> (3 + lg), grp = tid >> (3 + lg), j = (tid >> 3) & (sub - 1);
             for (int g0 = 0; g0 < ncol; g0 += ng) {
                 const bool on = g0 + grp < ncol;
-                const int k = S.lvl_cols[q0 + (on ? g0 + grp : 0)];
+                const int k = S.lvl_cols[p0 + (on ? g0 + grp : 0)];
                 const int blk = S.base[k];
-                double s = 0.0;
-                if (on) {
-                    int m = 0;
-                    for (int w = k >> 5; w < kSparseWords; ++w) m += __popc(S.colb[k * kSparseWords + w]);
-                    for (int a = 1 + j; a <= m; a += sub) {
-                        const double* Lb = S.L + 36LL * (blk + a) + c;
-                        double x[6];
-                        ld6(S.x + 6 * (S.ku[blk + a] & 255), x);
+                const int m = on ? S.height[k] - 1 : 0;
+                double r = j == 0 ? S.y[6 * k + c] : 0.0;
+#pragma unroll 2
+                for (int a = 1 + j; a <= m; a += sub) {
+                    const double* Lb = L + 36 * (blk + a) + e0;
+                    const double* x = S.y + 6 * ((S.desc[blk + a].y >> 24) & 255);
+                    double s = 0.0;
 #pragma unroll
-                        for (int r = 0; r < 6; ++r) s += Lb[6 * r] * x[r];
-                    }
+                    for (int p = 0; p < 6; ++p) s += Lb[es * p] * x[p];
+                    r -= s;
                 }
-                for (int o = 8; o < 8 * sub; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                const double r = S.y[6 * k + c] - s;
-                const double* Li = S.Linv + kInvStride * k;
-                double x = 0.0;
+                for (int o = 8; o < 8 * sub; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+                const double* D = L + 36 * blk;
+                double xs[6], x = 0.0;  // every lane: x = L_kk^-T r
 #pragma unroll
-                for (int p = 0; p < 6; ++p) {
-                    const double rp = __shfl_sync(0xffffffffu, r, p, 8);
-                    if (p >= c) x += Li[p * (p + 1) / 2 + c] * rp;
+                for (int p = 0; p < 6; ++p) xs[p] = __shfl_sync(0xffffffffu, r, p, 8);
+#pragma unroll
+                for (int p = 5; p >= 0; --p) {
+                    double t = xs[p];
+#pragma unroll
+                    for (int q = p + 1; q < 6; ++q) t -= D[frag(q, p)] * xs[q];
+                    xs[p] = t * D[frag(p, p)];
+                    if (p == c) x = xs[p];
                 }
-                if (on && j == 0 && cc < 6) {
-                    S.x[6 * k + cc] = x;
-                    B.du[6 * S.body[k] + cc] = x;
+                __syncwarp();
+                if (on && j == 0 && c8 < 6) {
+                    S.y[6 * k + c8] = x;
+                    B.du[6 * S.body[k] + c8] = x;
                 }
             }
             T.sync();
@@ -2273,7 +2501,7 @@ class SceneSolver {
                 for (int q = 0; q < 6; ++q) B.du[6 * gb + q] += (double)B.eF[6 * gb + q];
             }
             T.sync();
-            spmv_to_X(B.du, nullptr, 0.0);
+            spmv_to_X(B.du);
             T.sync();
             double s5[1] = {0};
             for (int i = tid; i < n_local; i += nt) {
@@ -2313,8 +2541,8 @@ class SceneSolver {
                 }
                 float pn[6];
                 for (int q = 0; q < 6; ++q) pn[q] = __fadd_rn(B.zF[6 * gb + q], __fmul_rn(beta, B.pF[6 * gb + q]));
-                const float cx = (float)B.arm[6 * gc + 3 * j], cy = (float)B.arm[6 * gc + 3 * j + 1],
-                            cz = (float)B.arm[6 * gc + 3 * j + 2];
+                const d3 ca = arm(contact(gc), j);
+                const float cx = (float)ca.x, cy = (float)ca.y, cz = (float)ca.z;
                 pv[j][0] = pn[0] + (pn[4] * cz - pn[5] * cy);
                 pv[j][1] = pn[1] + (pn[5] * cx - pn[3] * cz);
                 pv[j][2] = pn[2] + (pn[3] * cy - pn[4] * cx);
@@ -2340,8 +2568,8 @@ class SceneSolver {
             const int gc = e >> 1, side = e & 1;
             const float sg = side ? 1.f : -1.f;
             const float x = sg * B.Xf[3 * gc], y = sg * B.Xf[3 * gc + 1], z = sg * B.Xf[3 * gc + 2];
-            const float cx = (float)B.arm[6 * gc + 3 * side], cy = (float)B.arm[6 * gc + 3 * side + 1],
-                        cz = (float)B.arm[6 * gc + 3 * side + 2];
+            const d3 ca = fld3(incidence(st + k), I_arm);
+            const float cx = (float)ca.x, cy = (float)ca.y, cz = (float)ca.z;
             a[0] += x; a[1] += y; a[2] += z;
             a[3] += cy * z - cz * y; a[4] += cz * x - cx * z; a[5] += cx * y - cy * x;
         }
@@ -2356,24 +2584,25 @@ class SceneSolver {
         }
     }
 
-    // X = W (v1p - v0p) of direction vec (or of z + beta*vec when zvec != null),
-    // with the direction of static / non-active bodies taken as zero.
-    __device__ __forceinline__ void spmv_to_X(const double* vec, const double* zvec, double beta) const {
+    // X = W (v1p - v0p) of direction vec, with the direction of static /
+    // non-active bodies taken as zero.
+    __device__ __forceinline__ void spmv_to_X(const double* vec) const {
         for (int c = tid; c < nc; c += nt) {
             const int gc = c0 + c;
+            const double* P = contact(gc);
+            const int2 sl = reinterpret_cast<const int2*>(B.islot)[gc];
+            if (sl.x < 0 && sl.y < 0) continue;  // two static bodies
+            double W[6];
+            ld6(B.G + 12LL * max(sl.x, sl.y), W);  // both sides hold the contact's W
             d3 pv[2];
             for (int j = 0; j < 2; ++j) {
                 const int gb = b0 + B.cbody[2 * gc + j];
                 if (B.is_static[gb]) { pv[j] = d3{0, 0, 0}; continue; }
                 double pn[6];
-                if (zvec) {
-                    for (int r = 0; r < 6; ++r) pn[r] = __dadd_rn(zvec[6 * gb + r], __dmul_rn(beta, vec[6 * gb + r]));
-                } else {
-                    for (int r = 0; r < 6; ++r) pn[r] = vec[6 * gb + r];
-                }
-                pv[j] = point_vel(pn, ld3(B.arm + 6 * gc + 3 * j));
+                ld6(vec + 6LL * gb, pn);
+                pv[j] = point_vel(pn, arm(P, j));
             }
-            put_x(gc, sym_mul(B.W + 6 * gc, sub3(pv[1], pv[0])));
+            put_x(gc, sym_mul(W, sub3(pv[1], pv[0])));
         }
     }
     // (M/cm + eps I) x + gather(X)  for one active body
@@ -2397,18 +2626,20 @@ class SceneSolver {
         double a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0;
 #pragma unroll 2
         for (int k = 0; k < n; ++k) {
-            const int e = B.inc[st + k], go = B.inc_o[st + k];
-            const int gc = e >> 1, side = e & 1;
-            const d3 arm = ld3(B.arm + 6 * gc + 3 * side);
+            const int go = B.inc_o[st + k];
+            double W[12];
+            ldg12(st + k, W);
+            const d3 arm = ld3(W + 6);
             const d3 pv_own = point_vel(pn, arm);
             d3 pv_oth = d3{0, 0, 0};
             if (go >= 0) {
-                double po[6];
-                for (int r = 0; r < 6; ++r) po[r] = __dadd_rn(B.z[6 * go + r], __dmul_rn(beta, pp[6 * go + r]));
-                pv_oth = point_vel(po, ld3(B.arm + 6 * gc + 3 * (1 - side)));
+                double po[6], zo[6];
+                ld6(pp + 6LL * go, po);
+                ld6(B.z + 6LL * go, zo);
+                for (int r = 0; r < 6; ++r) po[r] = __dadd_rn(zo[r], __dmul_rn(beta, po[r]));
+                pv_oth = point_vel(po, ld3(W + 9));
             }
-            d3 x = sym_mul(B.W + 6 * gc, side ? sub3(pv_own, pv_oth) : sub3(pv_oth, pv_own));
-            if (!side) x = scl3(-1.0, x);
+            const d3 x = sym_mul(W, sub3(pv_own, pv_oth));  // sigma W (v1p - v0p)
             const d3 t = cross3(arm, x);
             a0 += x.x; a1 += x.y; a2 += x.z;
             a3 += t.x; a4 += t.y; a5 += t.z;
@@ -2459,18 +2690,20 @@ class SceneSolver {
         const int st = (gb >= 0) ? B.inc_start[gb] : 0, n = (gb >= 0) ? B.inc_cnt[gb] : 0;
 #pragma unroll 2
         for (int k = lg; k < n; k += L) {
-            const int e = B.inc[st + k], go = B.inc_o[st + k];
-            const int gc = e >> 1, side = e & 1;
-            const d3 arm = ld3(B.arm + 6 * gc + 3 * side);
+            const int go = B.inc_o[st + k];
+            double W[12];
+            ldg12(st + k, W);
+            const d3 arm = ld3(W + 6);
             const d3 pv_own = point_vel(pn, arm);
             d3 pv_oth = d3{0, 0, 0};
             if (go >= 0) {
-                double po[6];
-                for (int r = 0; r < 6; ++r) po[r] = __dadd_rn(B.z[6 * go + r], __dmul_rn(beta, pp[6 * go + r]));
-                pv_oth = point_vel(po, ld3(B.arm + 6 * gc + 3 * (1 - side)));
+                double po[6], zo[6];
+                ld6(pp + 6LL * go, po);
+                ld6(B.z + 6LL * go, zo);
+                for (int r = 0; r < 6; ++r) po[r] = __dadd_rn(zo[r], __dmul_rn(beta, po[r]));
+                pv_oth = point_vel(po, ld3(W + 9));
             }
-            d3 x = sym_mul(B.W + 6 * gc, side ? sub3(pv_own, pv_oth) : sub3(pv_oth, pv_own));
-            if (!side) x = scl3(-1.0, x);
+            const d3 x = sym_mul(W, sub3(pv_own, pv_oth));  // sigma W (v1p - v0p)
             const d3 t = cross3(arm, x);
             a0 += x.x; a1 += x.y; a2 += x.z;
             a3 += t.x; a4 += t.y; a5 += t.z;
@@ -2505,75 +2738,74 @@ class SceneSolver {
         }
     }
 
-    // filterLineSearch (NonSmoothContactForce.cpp:281-319) applied to step*d
-    __device__ __forceinline__ void filter(int gc, double step, double* dfin, double* dlin) const {
-        const double mu = cmu(gc);
-        const double cf0 = B.f[3 * gc], cf1 = B.f[3 * gc + 1], cf2 = B.f[3 * gc + 2];
-        dfin[0] = step * B.df[3 * gc];
-        dfin[1] = step * B.df[3 * gc + 1];
-        dfin[2] = step * B.df[3 * gc + 2];
-        double t0 = cf0 + dfin[0], t1 = cf1 + dfin[1], t2 = cf2 + dfin[2];
+    // filterLineSearch (NonSmoothContactForce.cpp:281-319) applied to step*d at
+    // force cf and multipliers l
+    __device__ __forceinline__ void filter(const double* P, double step, double mu, d3 cf, const double* l, double* dfin,
+                                           double* dlin) const {
+        const d3 d = fld3(P, F_df);
+        dfin[0] = step * d.x;
+        dfin[1] = step * d.y;
+        dfin[2] = step * d.z;
+        double t0 = cf.x + dfin[0], t1 = cf.y + dfin[1], t2 = cf.z + dfin[2];
         if (t0 < 0) {
             t0 = 0;
-            dfin[0] = t0 - cf0;
-            dfin[1] = t1 - cf1;
-            dfin[2] = t2 - cf2;
+            dfin[0] = t0 - cf.x;
+            dfin[1] = t1 - cf.y;
+            dfin[2] = t2 - cf.z;
         }
         if (cone_c(t0, t1, t2, mu) > 0) {
             // project(tf, tf) (LorentzCircleConstraint.cpp:36-49)
-            double o0 = t0, o1 = t1, o2 = t2;
-            if (t0 < 0) o0 = 0;
-            if (cone_c(o0, o1, o2, mu) > 0) {
-                const double rad = dmax(cone_radius(t0, mu) + 0, 0.0);
-                const double s = rad / sqrt(o1 * o1 + o2 * o2);
-                o1 *= s;
-                o2 *= s;
-            }
-            dfin[0] = o0 - cf0;
-            dfin[1] = o1 - cf1;
-            dfin[2] = o2 - cf2;
+            const double rad = dmax(cone_radius(t0, mu) + 0, 0.0);
+            const double s = rad / sqrt(__fma_rn(t2, t2, __dmul_rn(t1, t1)));
+            dfin[0] = t0 - cf.x;
+            dfin[1] = __dmul_rn(t1, s) - cf.y;
+            dfin[2] = __dmul_rn(t2, s) - cf.z;
         }
         for (int k = 0; k < 2; ++k) {
-            double d = step * B.dl[2 * gc + k];
-            const double l = B.lam[2 * gc + k];
-            if (d < 0 && l + d < 0) d = -l;
-            dlin[k] = d;
+            double e = step * P[32 * (F_dl + k)];
+            if (e < 0 && l[k] + e < 0) e = -l[k];
+            dlin[k] = e;
         }
     }
 
     // One contact of a line-search trial at `step` (filterLineSearch, the trial
     // point f + 0.99 df, lambda + 0.99 dl, and its residuals): trial values into
-    // fo / lo, the world impulse into the incidence slots xbuf; adds |wrf|^2,
+    // fo / lo, the world impulse into field xf of the incidence slots; adds |wrf|^2,
     // |rl|^2, |AC|^2 to q[1..3] and the directional terms to q[5], q[6].
-    __device__ __forceinline__ void trial_contact(int gc, double step, double muc, double* fo, double* lo,
-                                                  double* xbuf, double* q) const {
-        double dfin[3], dlin[2], fI[3], lI[2];
-        filter(gc, step, dfin, dlin);
-        for (int k = 0; k < 2; ++k) lI[k] = __dadd_rn(B.lam[2 * gc + k], __dmul_rn(0.99, dlin[k]));
-        for (int k = 0; k < 3; ++k) fI[k] = __dadd_rn(B.f[3 * gc + k], __dmul_rn(0.99, dfin[k]));
-        for (int k = 0; k < 3; ++k) fo[3 * gc + k] = fI[k];
-        for (int k = 0; k < 2; ++k) lo[2 * gc + k] = lI[k];
+    __device__ __forceinline__ void trial_contact(int gc, double step, double muc, int fo, int lo,
+                                                  int xf, double* q) const {
+        double* const P = contact(gc);
+        double dfin[3], dlin[2], lI[2];
+        const double l[2] = {P[32 * F_lam], P[32 * (F_lam + 1)]};
+        const d3 cf = fld3(P, F_f);
+        const double mu = cmu(gc);
+        filter(P, step, mu, cf, l, dfin, dlin);
+        for (int k = 0; k < 2; ++k) lI[k] = __dadd_rn(l[k], __dmul_rn(0.99, dlin[k]));
+        const d3 fI = d3{__dadd_rn(cf.x, __dmul_rn(0.99, dfin[0])), __dadd_rn(cf.y, __dmul_rn(0.99, dfin[1])),
+                         __dadd_rn(cf.z, __dmul_rn(0.99, dfin[2]))};
+        fst3(P, fo, fI);
+        for (int k = 0; k < 2; ++k) P[32 * (lo + k)] = lI[k];
         // residual at the trial point u + 0.99 step du: J is linear, so its
         // relative velocity is J u + 0.99 step J du (both stored per contact)
-        const Frame R = ld_frame(B.frame + 9 * gc);
         const double a = __dmul_rn(0.99, step);
-        const d3 wu = ld3(B.wu + 3 * gc), wd = ld3(B.wd + 3 * gc);
+        const d3 wu = fld3(P, F_wu), wd = fld3(P, F_wd);
         const d3 w = d3{fma(a, wd.x, wu.x), fma(a, wd.y, wu.y), fma(a, wd.z, wu.z)};
-        double rfv[3], rlv[2];
-        contact_residual_w(gc, R, w, fI, lI, muc, rfv, rlv, q[1], q[2], q[3], xbuf);
-        q[5] += dfin[0] * rfv[0] + dfin[1] * rfv[1] + dfin[2] * rfv[2];
+        d3 rf;
+        double rlv[2];
+        contact_residual_w(gc, P, w, fI, lI, mu, muc, rf, rlv, q[1], q[2], q[3], xf);
+        q[5] += dfin[0] * rf.x + dfin[1] * rf.y + dfin[2] * rf.z;
         q[6] += (dlin[0] / lI[0]) * rlv[0];
         if (!C.only_normal) q[6] += (dlin[1] / lI[1]) * rlv[1];
     }
     // One active body of a line-search trial: |ru|^2 at u + 0.99 step du into
     // q[0], du . ru into q[4]
-    __device__ __forceinline__ void trial_body(int gb, double step, const double* xbuf, double* q) const {
-        double ui[6], ruv[6];
-        trial_u(gb, step, ui);
-        double r2 = 0;
-        body_residual(gb, ui, ruv, r2, xbuf);
+    __device__ __forceinline__ void trial_body(int gb, double step, int xf, double* q) const {
+        double ui[6], d[6], v[6], r2 = 0;
+        trial_u(gb, step, ui, d);
+        body_residual(gb, ui, xf, v);
+        for (int r = 0; r < 6; ++r) r2 += v[r] * v[r];
         q[0] += r2;
-        for (int r = 0; r < 6; ++r) q[4] += (step * B.du[6 * gb + r]) * ruv[r];
+        for (int r = 0; r < 6; ++r) q[4] += (step * d[r]) * v[r];
     }
     // Acceptance of trial t (lineSearch :606-630): 1 = accept, 2 = stop without
     // a step (the last trial failed), 0 = halve the step and go on.
@@ -2586,18 +2818,18 @@ class SceneSolver {
         return 0;
     }
     // Commit of an accepted trial at `step` with trial values fo / lo
-    __device__ __forceinline__ void ls_commit(double step, const double* fo, const double* lo) {
+    __device__ __forceinline__ void ls_commit(double step, int fo, int lo) {
         for (int i = tid; i < n_local; i += nt) {
             const int gb = B.lbody[b0 + i];
-            if (!B.local[gb]) continue;
-            double ui[6];
-            trial_u(gb, step, ui);
-            for (int r = 0; r < 6; ++r) B.u[6 * gb + r] = ui[r];
+            double ui[6], d[6];
+            trial_u(gb, step, ui, d);
+            st6(B.u + 6LL * gb, ui);
         }
         for (int c = tid; c < nc; c += nt) {
             const int gc = c0 + c;
-            for (int k = 0; k < 3; ++k) B.f[3 * gc + k] = fo[3 * gc + k];
-            for (int k = 0; k < 2; ++k) B.lam[2 * gc + k] = lo[2 * gc + k];
+            double* const P = contact(gc);
+            for (int k = 0; k < 3; ++k) P[32 * (F_f + k)] = P[32 * (fo + k)];
+            for (int k = 0; k < 2; ++k) P[32 * (F_lam + k)] = P[32 * (lo + k)];
         }
         T.sync();
     }
@@ -2617,9 +2849,7 @@ class SceneSolver {
         if constexpr (Team::kind == 0) {
           if (nc <= half && n_local <= half) {
             const int j = tid >= half ? 1 : 0, k = tid - j * half;
-            double* fo = j ? B.fT2 : B.fT;
-            double* lo = j ? B.lT2 : B.lT;
-            double* xo = j ? B.Xi2 : B.Xi;
+            const int fo = j ? F_fT2 : F_fT, lo = j ? F_lT2 : F_lT, xo = j ? I_X2 : I_X;
             for (int t = 0; t < maxLS; t += 2) {
                 const double sj = j ? step * 0.5 : step;
                 double q[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -2638,12 +2868,12 @@ class SceneSolver {
                 T.sum(e);
                 ++trials;
                 int v = ls_verdict(e, sErr, sacErr, t, maxLS);
-                if (v == 1) { ls_commit(step, B.fT, B.lT); return step; }
+                if (v == 1) { ls_commit(step, F_fT, F_lT); return step; }
                 if (v == 2) break;
                 if (t + 1 >= maxLS) break;
                 ++trials;
                 v = ls_verdict(e + 7, sErr, sacErr, t + 1, maxLS);
-                if (v == 1) { ls_commit(step * 0.5, B.fT2, B.lT2); return step * 0.5; }
+                if (v == 1) { ls_commit(step * 0.5, F_fT2, F_lT2); return step * 0.5; }
                 if (v == 2) break;
                 step *= 0.25;
             }
@@ -2653,60 +2883,41 @@ class SceneSolver {
         for (int t = 0; t < maxLS; ++t) {
             ++trials;
             double e[7] = {0, 0, 0, 0, 0, 0, 0};  // ru2, wrf2, rl2, ac2, du.ru, df.rf, (dl/l).rl
-            for (int c = tid; c < nc; c += nt) trial_contact(c0 + c, step, muc, B.fT, B.lT, B.Xi, e);
+            for (int c = tid; c < nc; c += nt) trial_contact(c0 + c, step, muc, F_fT, F_lT, I_X, e);
             T.sync();
             for (int i = tid; i < n_local; i += nt) {
                 const int gb = B.lbody[b0 + i];
-                if (!active(gb)) continue;
-                trial_body(gb, step, B.Xi, e);
+                if (active(gb)) trial_body(gb, step, I_X, e);
             }
             T.sum(e);
             const int v = ls_verdict(e, sErr, sacErr, t, maxLS);
-            if (v == 1) { ls_commit(step, B.fT, B.lT); return step; }
+            if (v == 1) { ls_commit(step, F_fT, F_lT); return step; }
             if (v == 2) break;
             step *= 0.5;
         }
         return 0.0;
     }
-    __device__ __forceinline__ void trial_u(int gb, double step, double* ui) const {
-        for (int r = 0; r < 6; ++r)
-            ui[r] = __dadd_rn(B.u[6 * gb + r], __dmul_rn(0.99, __dmul_rn(step, B.du[6 * gb + r])));
+    __device__ __forceinline__ void trial_u(int gb, double step, double* ui, double* d) const {
+        ld6(B.u + 6LL * gb, ui);
+        ld6(B.du + 6LL * gb, d);
+        for (int r = 0; r < 6; ++r) ui[r] = __dadd_rn(ui[r], __dmul_rn(0.99, __dmul_rn(step, d[r])));
     }
     // contact residual with fresh constraints, given the relative velocity w
-    __device__ __forceinline__ void contact_residual_w(int gc, const Frame& R, d3 w, const double* fv,
-                                                       const double* lv, double muc, double* rfo, double* rlo,
-                                                       double& wrf2, double& rl2, double& ac2, double* xbuf = nullptr) const {
+    __device__ __forceinline__ void contact_residual_w(int gc, const double* P, d3 w, d3 fv, const double* lv, double mu, double muc,
+                                                       d3& rfo, double* rlo, double& wrf2, double& rl2, double& ac2,
+                                                       int xf) const {
+        const Frame R = frame(P);
         if (C.only_normal) {
-            normal_residual(gc, R, w, fv[0], lv[0], muc, rfo, rlo, wrf2, rl2, ac2, xbuf);
+            rlo[1] = 0;
+            normal_residual(gc, P, R, w, fv.x, lv[0], muc, rfo, rlo[0], wrf2, rl2, ac2, xf);
             return;
         }
-        const double fn = fv[0], f1 = fv[1], f2 = fv[2];
-        const double mu = cmu(gc);
         double g0, g1;
-        cone_grad(f1, f2, g0, g1);
-        double r0 = 0 - w.x, r1 = 0 - w.y, r2 = 0 - w.z;
-        if (C.spring_based) r0 -= compliance * cm * fn;
-        r0 += lv[0];
-        r1 -= lv[1] * g0;
-        r2 -= lv[1] * g1;
-        r0 -= B.kn[gc];
-        const double rl0 = lv[0] * (-fn) + muc, rl1 = lv[1] * cone_c(fn, f1, f2, mu) + muc;
-        const double wt = tangential_weight(gc, R, w, fn);
-        const double w1 = r1 * wt, w2 = r2 * wt;
-        wrf2 += r0 * r0 + w1 * w1 + w2 * w2;
+        cone_grad(fv.y, fv.z, g0, g1);
+        const double rl0 = lv[0] * (-fv.x) + muc, rl1 = lv[1] * cone_c(fv.x, fv.y, fv.z, mu) + muc;
         rl2 += rl0 * rl0 + rl1 * rl1;
-        const double tp = fn - (w.x + B.kn[gc] + spring_term * fn);
-        const double a0 = dmax(tp, 0.0) - fn;
-        const double rad = cone_radius(fn, mu);
-        const double td0 = f1 - w.y, td1 = f2 - w.z;
-        const double tdn = sqrt(td0 * td0 + td1 * td1);
-        double p0 = td0, p1 = td1;
-        if (!(tdn < rad)) { p0 = td0 * rad / tdn; p1 = td1 * rad / tdn; }
-        const double a1 = p0 - f1, a2 = p1 - f2;
-        ac2 += a0 * a0 + a1 * a1 + a2 * a2;
-        rfo[0] = r0; rfo[1] = r1; rfo[2] = r2;
+        rfo = cone_residual(gc, P, R, w, fv, lv[0], lv[1], g0, g1, mu, wrf2, ac2, xf);
         rlo[0] = rl0; rlo[1] = rl1;
-        put_x(gc, scl3(-1.0, from_frame(R, d3{fn, f1, f2})), xbuf);
     }
 
     // KKT report at the final iterate (mu_c = 0) and write-back (:491-510).
@@ -2715,24 +2926,32 @@ class SceneSolver {
         double mx[2] = {0, 0};
         for (int c = tid; c < nc; c += nt) {
             const int gc = c0 + c;
-            const Frame R = ld_frame(B.frame + 9 * gc);
-            const d3 w = rel_vel(gc, B.u);
-            double rfv[3], rlv[2], d1 = 0, d2 = 0, d3v = 0;
-            contact_residual_w(gc, R, w, B.f + 3 * gc, B.lam + 2 * gc, 0.0, rfv, rlv, d1, d2, d3v);
-            e[1] += rfv[0] * rfv[0] + rfv[1] * rfv[1] + rfv[2] * rfv[2];
+            double* const P = contact(gc);
+            const d3 w = rel_vel(gc, P, B.u), fv = fld3(P, F_f);
+            const double l[2] = {P[32 * F_lam], P[32 * (F_lam + 1)]};
+            const double mu = cmu(gc);
+            d3 rf;
+            double rlv[2], d1 = 0, d2 = 0, d3v = 0;
+            contact_residual_w(gc, P, w, fv, l, mu, 0.0, rf, rlv, d1, d2, d3v, I_X);
+            e[1] += dot3(rf, rf);
             mx[0] = dmax(mx[0], dmax(fabs(rlv[0]), fabs(rlv[1])));
-            const double fn = B.f[3 * gc];
-            mx[1] = dmax(mx[1], C.only_normal ? -fn : dmax(-fn, cone_c(fn, B.f[3 * gc + 1], B.f[3 * gc + 2], cmu(gc))));
-            for (int k = 0; k < 3; ++k) B.lforce[3 * gc + k] = B.f[3 * gc + k] * cs * cm;
+            mx[1] = dmax(mx[1], C.only_normal ? -fv.x : dmax(-fv.x, cone_c(fv.x, fv.y, fv.z, mu)));
+            B.lforce[3 * gc] = fv.x * cs * cm;
+            B.lforce[3 * gc + 1] = fv.y * cs * cm;
+            B.lforce[3 * gc + 2] = fv.z * cs * cm;
         }
         T.sync();
         for (int i = tid; i < n_local; i += nt) {
             const int gb = B.lbody[b0 + i];
-            if (!B.local[gb]) continue;
-            if (!B.is_static[gb]) body_residual(gb, B.u + 6 * gb, nullptr, e[0]);
+            double ub[6], v[6];
+            ld6(B.u + 6LL * gb, ub);
+            if (!B.is_static[gb]) {
+                body_residual(gb, ub, I_X, v);
+                for (int r = 0; r < 6; ++r) e[0] += v[r] * v[r];
+            }
             for (int r = 0; r < 3; ++r) {
-                B.dvel[3 * gb + r] = B.u[6 * gb + r] * cs - B.vel[3 * gb + r];
-                B.dang[3 * gb + r] = B.u[6 * gb + 3 + r] * cs - B.ang[3 * gb + r];
+                B.dvel[3 * gb + r] = ub[r] * cs - B.vel[3 * gb + r];
+                B.dang[3 * gb + r] = ub[3 + r] * cs - B.ang[3 * gb + r];
             }
         }
         T.sum(e);
@@ -2865,10 +3084,9 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) solve_scenes_kernel(co
                                                            const __grid_constant__ EngineCfg C) {
     __shared__ double s_red[2 * 16 * 32];
     __shared__ int s_int[33];
-    __shared__ uint32_t s_adj[kSparseMax * kSparseWords];
     __shared__ int s_q;
     {
-        CtaTeam T(s_red, s_int, s_adj);
+        CtaTeam T(s_red, s_int);
         const int n_cta = B.counts[0];
         for (;;) {
             if (threadIdx.x == 0) s_q = atomicAdd(&B.counts[2], 1);
