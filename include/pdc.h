@@ -118,7 +118,9 @@ typedef struct pdc_config {
     int32_t cluster_max_bodies; /* (4096) */
     int32_t pcg_lanes;         /* lanes per body in the PCG product: 1, 2, 4 or 8 (0 = 1 for
                                   block and warp teams, 4 for the large-scene teams) */
-    double pcg_rtol_direct;   /* PCG relative residual standing in for LDLT (1e-13) */
+    double pcg_rtol_direct;   /* PCG relative residual (the recurrence's) standing in for LDLT (1e-15;
+                                 at 1e-13 velocities can be 1e-5 away from a direct solve's).
+                                 Mixed precision refines its true residual to no less than 1e-13 */
     int32_t pcg_max_direct;   /* PCG iteration cap on the direct branch (4000) */
     double pcg_rtol_iter;     /* relative residual of the iterative branch (1e-8, AMGCL's) */
     int32_t pcg_max_iter;     /* iteration cap of the iterative branch (1000, :381) */

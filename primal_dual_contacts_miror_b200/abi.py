@@ -219,7 +219,7 @@ def default_config(**overrides):
     cfg.cluster_max_contacts = 4096
     cfg.cluster_max_bodies = 4096
     cfg.pcg_lanes = 0
-    cfg.pcg_rtol_direct = 1e-13
+    cfg.pcg_rtol_direct = 1e-15
     cfg.pcg_max_direct = 4000
     cfg.pcg_rtol_iter = 1e-8
     cfg.pcg_max_iter = 1000

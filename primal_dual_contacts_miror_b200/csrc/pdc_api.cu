@@ -317,7 +317,7 @@ extern "C" void pdc_config_default(pdc_config* c) {
     c->cluster_max_contacts = 4096;
     c->cluster_max_bodies = 4096;
     c->pcg_lanes = 0;
-    c->pcg_rtol_direct = 1e-13;
+    c->pcg_rtol_direct = 1e-15;
     c->pcg_max_direct = 4000;
     c->pcg_rtol_iter = 1e-8;
     c->pcg_max_iter = 1000;  // :381

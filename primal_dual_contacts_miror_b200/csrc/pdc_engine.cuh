@@ -145,6 +145,11 @@ struct BatchPtrs {
 
 #define PDC_STATUS_BAD_INPUT 16
 
+// Mixed precision tests its stop on the true residual in FP64, which rounding keeps
+// above ~1e-14 |b|; the FP64 PCG's recurrence residual goes on below that (and has
+// to: where the matrix is soft, stopping it at 1e-13 |b| leaves velocities 1e-5 off).
+constexpr double kMixedRtolMin = 1e-13;
+
 // Per-contact workspace: tiles of 32 contacts, one run of 32 values per field, so
 // that a warp's loads and stores are coalesced and every field of a contact is
 // a constant offset from one address.  (With a contact's components side by
@@ -954,7 +959,7 @@ class SceneSolver {
             bool fp64_pcg = !dense_mode;
             if (!dense_mode && C.mixed) {
                 bool conv = true;
-                const bool ok = mixed_solve(eps, bnorm, rtol, iters, conv);
+                const bool ok = mixed_solve(eps, bnorm, dmax(rtol, kMixedRtolMin), iters, conv);
                 pcg_total += iters;
                 iters = 0;
                 fp64_pcg = !(ok && conv);
