@@ -895,16 +895,13 @@ class SceneSolver {
                     const d3 c = ld3(W + 6);
                     // Y = C W (C = [c]x): column k of Y = c x W_col_k
                     const d3 wc0 = d3{W[0], W[3], W[4]}, wc1 = d3{W[3], W[1], W[5]}, wc2 = d3{W[4], W[5], W[2]};
-                    // (roundings spelled out; the y as in assemble_rows)
+                    // (rounded as assemble_rows rounds the factor's diagonal blocks)
                     const d3 y0 = cross_rn(c, wc0), y2 = cross_rn(c, wc2);
                     d3 y1 = cross_rn(c, wc1);
                     y1.y = __fma_rn(-c.x, wc1.z, __dmul_rn(c.z, wc1.x));
                     // Z = C Y^T: column k of Z = c x (row k of Y)
-                    d3 z0 = cross_rn(c, d3{y0.x, y1.x, y2.x});
-                    d3 z1 = cross_rn(c, d3{y0.y, y1.y, y2.y});
-                    z0.y = __fma_rn(-c.x, y2.x, __dmul_rn(c.z, y0.x));
-                    z0.z = __fma_rn(-c.y, y0.x, __dmul_rn(c.x, y1.x));
-                    z1.z = __fma_rn(-c.y, y0.y, __dmul_rn(c.x, y1.y));
+                    const d3 z0 = cross_rn(c, d3{y0.x, y1.x, y2.x});
+                    const d3 z1 = cross_rn(c, d3{y0.y, y1.y, y2.y});
                     const d3 z2 = cross_rn(c, d3{y0.z, y1.z, y2.z});
                     P[pk(0, 0)] += W[0]; P[pk(1, 0)] += W[3]; P[pk(1, 1)] += W[1];
                     P[pk(2, 0)] += W[4]; P[pk(2, 1)] += W[5]; P[pk(2, 2)] += W[2];
