@@ -92,13 +92,14 @@ struct BlockReducer {
     int parity;
     __device__ void init(double* s) { slots = s; parity = 0; }
     // The warp stage halves the values with every exchange (lanes that differ in
-    // bit 4 keep one half of the values each, and so on), so M <= 8 sums take 9
-    // shuffles of doubles instead of 5 M, and M <= 16 take 17; then lane l adds
-    // the warps' slots of value l (both in the order of a plain shuffle tree).
+    // bit 4 keep one half of the values each, and so on) until a lane has one, then
+    // sums it over the lane bits that are left: 5 shuffles of doubles for M <= 2
+    // sums, 6 for M <= 4, 9 for M <= 8 and 16 for M <= 16, instead of 5 M; then lane
+    // l adds the warps' slots of value l (both in the order of a plain shuffle tree).
     template <int M>
     __device__ __forceinline__ void sum(double (&v)[M]) {
         static_assert(M <= N && M <= 16, "reduction wider than the slots");
-        constexpr int K = M <= 8 ? 8 : 16;
+        constexpr int K = M == 1 ? 1 : M == 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
         double* b = slots + parity * N * 32;
         parity ^= 1;
@@ -117,7 +118,7 @@ struct BlockReducer {
             }
             if (up) idx += h;
         }
-        constexpr int left = K == 8 ? 2 : 1;  // lane bits not yet summed over
+        constexpr int left = 16 / K;  // highest lane bit not yet summed over
 #pragma unroll
         for (int o = left; o >= 1; o >>= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
         if ((lane & (2 * left - 1)) == 0) b[warp * K + idx] = x[0];
