@@ -2026,7 +2026,6 @@ class SceneSolver {
     // product is the forward substitution's part.  One entry is 6 cycles of the
     // load-store unit; a thread per block row, loading its factor's 36 values
     // again for every row, took 29.
-    template <bool SM>
     __device__ __forceinline__ void update_block(const Direct& S, double* L, int i, int4 de, bool listed,
                                                  int lane) const {
         const int row = lane >> 2, kk = lane & 3, n = de.y & 0xffff;
@@ -2131,8 +2130,10 @@ class SceneSolver {
     // blocks) and no barrier but the level's.  Levels of short lists and patterns
     // (stacks, columns, loose piles) sum entry by entry in elimination order.
     // Long lists run on the FP64 matrix instruction: it has the rate of the FP64
-    // pipe, but feeds 256 multiply-adds from two loads per lane.  Stands in for
-    // the direct branch's SimplicialLDLT (:385-394).  Writes du; false on a
+    // pipe, but feeds 256 multiply-adds from two loads per lane, wherever the blocks
+    // are (in global memory, a thread per row instead: crate of 144 cubes 5.85 ->
+    // 7.51 ms, 1,024 crates of up to 216 12.8 -> 16.9 ms).  Stands in for the
+    // direct branch's SimplicialLDLT (:385-394).  Writes du; false on a
     // non-SPD pivot, which only marks the scene: later columns then compute
     // garbage in bounded loops.
     template <bool SM>
@@ -2155,7 +2156,7 @@ class SceneSolver {
                 } else {
                     for (int i = i0 + warp; i < i1; i += nwarp) {
                         const int4 de = S.desc[i];
-                        if ((de.y & 0xffff) != 0) update_block<SM>(S, L, i, de, listed, lane);
+                        if ((de.y & 0xffff) != 0) update_block(S, L, i, de, listed, lane);
                     }
                 }
                 T.sync();
