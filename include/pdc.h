@@ -98,7 +98,7 @@ typedef struct pdc_config {
     int32_t direct_threshold; /* local bodies below this use the direct-solve branch (2000) */
     int32_t sparse_max_bodies; /* direct branch: sparse block Cholesky on the device up to
                                   this many active bodies (256, the maximum; a batch of
-                                  many scenes holds one 9.7 MB factor slot per thread
+                                  many scenes holds one 10.1 MB factor slot per thread
                                   block in flight, enough for any factor); larger
                                   scenes use PCG */
     int32_t sparse_max_bodies_large; /* the same for scenes solved by a thread-block cluster
@@ -106,7 +106,8 @@ typedef struct pdc_config {
     int32_t warp_max_contacts; /* batched launch: scenes with at most this many contacts */
     int32_t warp_max_bodies;   /* and bodies are solved by one warp, larger ones by a
                                   whole thread block (0 / 0 = blocks only, the default;
-                                  at most 64 bodies when warp teams are on) */
+                                  at most 64 bodies when warp teams are on, which
+                                  hold a 0.74 MB factor slot per warp in flight) */
     int32_t cta_threads;       /* threads per block of the solve kernel: 128 or 256 (256) */
     int32_t grid_min_bodies;   /* scenes with at least this many bodies are large: solved one
                                   launch each, by a thread-block cluster or the whole GPU

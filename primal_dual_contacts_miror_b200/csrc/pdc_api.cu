@@ -26,14 +26,10 @@ thread_local std::string g_create_error;
 std::atomic<int> g_fail_allocs{0};
 constexpr int kThreads = 256;
 constexpr int kWarpsPerBlock = kThreads / 32;
-// sparse scratch of a thread-block team: bitsets, orders, offsets, 2x256
-// diagonal blocks, 4 node vectors, then room for any factor of 256 nodes
-constexpr long long kSparseHeaderDoubles = (pdc::kSparseHeaderBytes + 255) / 256 * 32;
-constexpr long long kSparseBlocks = pdc::kRowCap;  // off-diagonal L blocks per scene
-// a warp team's slot: the same fixed part, room for kWarpSparseBlocks blocks
-// (warp teams take scenes of at most kWarpMaxBodies bodies)
-constexpr int kWarpMaxBodies = 64;
-constexpr long long kWarpSparseBlocks = kWarpMaxBodies * (kWarpMaxBodies - 1) / 2;
+// sparse scratch of a thread-block team, with room for any factor of 256 nodes, and
+// of a warp team, with room for any factor of 64: 10.1 and 0.74 MB
+constexpr long long kSparseSlot = pdc::sparse_header_doubles(pdc::kRowCap) + 36LL * pdc::kRowCap;
+constexpr long long kSparseSlotWarp = pdc::sparse_header_doubles(pdc::kRowCapWarp) + 36LL * pdc::kRowCapWarp;
 // large-scene teams: index arrays, node blocks and kRowCapLarge off-diagonal blocks
 constexpr long long kSparseBigDoubles = pdc::kSparseLargeHeaderDoubles + 36LL * pdc::kRowCapLarge;
 
@@ -226,10 +222,10 @@ static size_t carve(Arena& A, int ns, long long nb, long long nc, pdc::BatchPtrs
     if (dense_max > 0) {
         // sparse factorisation scratch: one slot per thread block, and one per
         // warp when warp teams are on
-        P->dense_stride = kSparseHeaderDoubles + 36LL * kSparseBlocks;
+        P->dense_stride = kSparseSlot;
         P->dense = D((size_t)grid * P->dense_stride);
         if (warp_teams) {
-            P->dense_stride_warp = kSparseHeaderDoubles + 36LL * kWarpSparseBlocks;
+            P->dense_stride_warp = kSparseSlotWarp;
             P->dense_warp = D((size_t)grid * kWarpsPerBlock * P->dense_stride_warp);
         }
     }
@@ -341,7 +337,7 @@ static int validate_config(pdc_solver* s, const pdc_config* c) {
     if (c->mu_pair_hi > c->mu_pair_lo && !(c->mu_pair_lo >= 0)) return fail(s, PDC_EINVAL, "negative mu_pair_lo");
     if (c->pcg_lanes != 0 && c->pcg_lanes != 1 && c->pcg_lanes != 2 && c->pcg_lanes != 4 && c->pcg_lanes != 8)
         return fail(s, PDC_EINVAL, "pcg_lanes not in {0, 1, 2, 4, 8}");
-    if (c->warp_max_contacts > 0 && c->warp_max_bodies > kWarpMaxBodies)
+    if (c->warp_max_contacts > 0 && c->warp_max_bodies > pdc::kWarpMaxBodies)
         return fail(s, PDC_EINVAL, "warp_max_bodies above 64");
     if (c->sparse_max_bodies < 0 || c->sparse_max_bodies > pdc::kSparseMax)
         return fail(s, PDC_EINVAL, "sparse_max_bodies out of [0, 256]");
@@ -841,9 +837,8 @@ extern "C" void pdc_host_free(void* p) {
 // Limits: at most kNoAllocMaxBodies bodies and kNoAllocMaxContacts contacts
 // per call; larger scenes are rejected with PDC_EINVAL.  The array holds the
 // solver arrays of a scene at those limits plus one full sparse-factor slot
-// (the same kSparseBlocks off-diagonal blocks a handle gives each team), so a
-// scene inside the limits takes the same branch as in pdc_solve.  Every GPU
-// that loads the library holds the 12 MiB array until the process exits.  All
+// (kSparseSlot, as a handle gives each team), so a scene inside the limits takes
+// the same branch as in pdc_solve.  Every GPU that loads the library holds the 12 MiB array until the process exits.  All
 // calls share it and it keeps the last call's contents: the planner kernel
 // resets the work counters and each solve initialises every scratch value it
 // reads, so nothing needs clearing between calls -- but calls that overlap on
@@ -856,7 +851,7 @@ extern "C" void pdc_host_free(void* p) {
 namespace {
 constexpr int kNoAllocMaxBodies = 256;
 constexpr int kNoAllocMaxContacts = 2048;
-constexpr long long kNoAllocSparseDoubles = kSparseHeaderDoubles + 36LL * kSparseBlocks;  // one team slot
+constexpr long long kNoAllocSparseDoubles = kSparseSlot;  // one team slot
 constexpr long long kNoAllocDoubles = 1572864;                                             // 12 MiB
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;

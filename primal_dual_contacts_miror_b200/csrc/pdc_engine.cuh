@@ -195,14 +195,17 @@ constexpr int kSparseWords = kSparseMax / 32;
 // the direct branch never leaves the factor for lack of room (a settled heap of
 // 256 boxes fills in to several thousand blocks)
 constexpr int kRowCap = kSparseMax * (kSparseMax - 1) / 2;
-// 6x6 blocks of a factor: the off-diagonal ones and a diagonal one per node
-constexpr int kBlockCap = kRowCap + kSparseMax;
-// bytes of a slot before its blocks (bitsets, index arrays, block descriptors
-// and the node vector; the layout of SceneSolver::direct_ws), plus the diagonal
-// blocks and two spare ones (a zero block and room to read past the last)
-constexpr long long kSparseHeaderBytes = 4LL * (3LL * kSparseMax * kSparseWords + 12LL * (kSparseMax + 8)) +
-                                         16LL * (kBlockCap + 2) +
-                                         8LL * (6 * (kSparseMax + 2) + 36 * (kSparseMax + 2));
+// the same for a warp team, which takes scenes of at most kWarpMaxBodies bodies
+constexpr int kWarpMaxBodies = 64;
+constexpr int kRowCapWarp = kWarpMaxBodies * (kWarpMaxBodies - 1) / 2;
+// doubles of a slot before its off-diagonal blocks: bitsets, index arrays, block
+// descriptors and the node vector (the layout of SceneSolver::direct_ws), then the
+// diagonal blocks, one per node, and two spare ones (a zero block and room to read
+// past the last)
+__host__ __device__ constexpr long long sparse_header_doubles(int off_diagonal) {
+    return (4LL * (3LL * kSparseMax * kSparseWords + 12LL * (kSparseMax + 8)) + 16LL * (off_diagonal + kSparseMax + 2) +
+            8LL * (6 * (kSparseMax + 2) + 36 * (kSparseMax + 2)) + 255) / 256 * 32;
+}
 // Levels whose update lists (column patterns) have at most this many entries
 // are updated by a thread per row (substituted backward entry by entry).
 constexpr int kShortList = 4;
@@ -1275,7 +1278,8 @@ class SceneSolver {
         constexpr int M8 = kSparseMax + 8;
         Direct S;
         int4* d = reinterpret_cast<int4*>(first);
-        S.desc = d; d += kBlockCap + 2;
+        constexpr int cap = Team::kind == 1 ? kRowCapWarp : kRowCap;
+        S.desc = d; d += cap + kSparseMax + 2;
         double* v = reinterpret_cast<double*>(d);
         S.y = v; v += 6 * (kSparseMax + 2);
         int* q = reinterpret_cast<int*>(v);
@@ -1294,7 +1298,7 @@ class SceneSolver {
         S.lvl_len = q; q += M8;
         S.lvl_pat = q; q += M8;
         S.meta = q;
-        S.slot = first + (kSparseHeaderBytes + 255) / 256 * 32 - 36LL * (kSparseMax + 2);
+        S.slot = first + sparse_header_doubles(cap) - 36LL * (kSparseMax + 2);
         S.cap = (int)((stride - (S.slot - first)) / 36) - 2;
         S.L = S.slot;
         if constexpr (Team::kind == 0) S.y = block_smem();

@@ -107,3 +107,23 @@ def test_warp_teams():
                 b0, b1 = b0 + s.n_bodies, b1 + s.n_contacts
                 assert rel(lf[k * len(olf) + a1:k * len(olf) + b1], olf[a1:b1]) < 1e-9, (team, q)
                 assert rel(v[k * len(o) + a0:k * len(o) + b0], o[a0:b0], 0.0981) < 1e-9, (team, q)
+
+
+@pytest.mark.gpu
+def test_warp_slots_hold_factors_of_64():
+    """Device memory of a call with warp teams: a warp's slot has room for the blocks,
+    descriptors and lists of 64 bodies, no more than 0.92 MB (it once held descriptors
+    for every block of a 256-body factor, 1.23 MB); with 64 MB for everything else."""
+    import torch
+
+    from primal_dual_contacts_miror_b200 import lib
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    grid = 2 * sms  # blocks in flight, eight warps each
+    b = abi.HostBatch([scenes.settled_pile(2, np.random.default_rng(0))] * grid, 0.01, (0, 0, -9.81))
+    solver = lib.Solver(abi.default_config(warp_max_contacts=64, warp_max_bodies=64))
+    free = torch.cuda.mem_get_info()[0]
+    st = solver.batch_solve(b)[3]
+    used = free - torch.cuda.mem_get_info()[0]
+    assert all(s["team"] == 1 for s in st)
+    assert used < grid * (10.1e6 + 8 * 0.92e6) + 64e6, used
