@@ -83,8 +83,8 @@ __device__ __forceinline__ double cone_radius(double fn, double mu) {
 
 // ------------------------------------------- deterministic block reductions
 // Every thread passes its partial sums; every thread receives the identical
-// total (fixed tree: warp shuffle-down to lane 0, per-warp slots, then the same
-// tree over the slots in every warp).  `buf` alternates between two halves so a
+// total (fixed tree over the lanes of a warp, per-warp slots, then the same tree
+// over the slots in every warp).  `slots` alternates between two halves so a
 // single __syncthreads per reduction suffices.
 template <int N>
 struct BlockReducer {

@@ -8,12 +8,14 @@
 // (src/Solver/PrimalDual/PrimalDualForceSolver.cpp:167-511) with
 // NonSmoothContactForce (src/Solver/PrimalDual/NonSmoothForces/NonSmoothContactForce.cpp:8-319).
 // Differences in mechanism, not in the solution:
-//  * the 6N_b x 6N_b Newton system is never assembled; its product with a
-//    vector is applied matrix-free per contact (W = R K^-1 R^T, 6 doubles) and
-//    gathered per body;
-//  * the LDL^T / AMGCL solve (:385-427) is a block-Jacobi preconditioned CG,
-//    converged to cfg.rtol_direct (direct branch) or cfg.rtol_iter with the
-//    reference's AMGCL cap and Hu rule (iterative branch, >= 2000 local bodies);
+//  * the LDL^T solve (:385-394, < 2000 local bodies) is a sparse Cholesky
+//    factorisation of 6x6 body blocks, assembled from the contacts' W = R K^-1 R^T
+//    (6 doubles), up to 256 active bodies (block and warp teams) or 2048 (large
+//    teams, unless the factor would be too deep);
+//  * above that, and in place of AMGCL (:395-427), the system is never assembled:
+//    block-Jacobi preconditioned CG, the product applied per contact and gathered
+//    per body, converged to cfg.rtol_direct (direct branch) or cfg.rtol_iter with
+//    the reference's AMGCL cap and Hu rule (iterative branch);
 //  * the contact->body scatter, which the reference does with omp atomics
 //    (NonSmoothContactForce.cpp:144,228,243), is a gather over per-body
 //    incidence lists sorted by contact index, so results are bitwise
