@@ -55,10 +55,10 @@ SEED = 20241203 + 3 * 10 ** 6  # the batched workload's seed
 DT = 0.01
 GRAVITY = (0.0, 0.0, -9.81)
 # DRAM bytes of one solve_scenes_kernel launch on this workload: ncu's
-# dram__bytes of one launch on 1,024 box-drop scenes at world step 250 (31.5 GB;
+# dram__bytes of one launch on 1,024 box-drop scenes at world step 250 (17.5 GB;
 # the 4,096-scene world is above the capture size rule), scaled by the scene
 # count to a 4,096-scene launch (profiles/solve_scenes_kernel_boxdrops4096.md)
-TRAFFIC_PER_LAUNCH = 31.48e9 * 4
+TRAFFIC_PER_LAUNCH = 17.48e9 * 4
 
 
 def algorithmic_bytes(stats):

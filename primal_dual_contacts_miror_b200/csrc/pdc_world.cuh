@@ -41,8 +41,8 @@ __global__ void prepare_bodies_kernel(const __grid_constant__ WorldPtrs W, const
 // local memory) is what the time goes to: it runs once per candidate, with all
 // lanes on candidates, where a contiguous range of pairs per thread left most lanes
 // idle and needed a second pass for the offsets.  128 threads, since the narrow
-// phase takes nearly all registers a thread can have: two blocks per SM, and small
-// scenes leave fewer lanes idle than with 256.
+// phase takes 165 registers: three blocks per SM (their shared memory allows as
+// many), and small scenes leave fewer lanes idle than with 256.
 constexpr int kCollideThreads = 128;
 constexpr int kPairRounds = 4;       // AABB tests per thread between two barriers
 constexpr int kCollideBodies = 512;  // bodies whose boxes are kept in shared memory
