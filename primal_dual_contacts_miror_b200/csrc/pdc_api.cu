@@ -952,8 +952,9 @@ extern "C" int pdc_solve_noalloc(const pdc_config* cfg, double dt, const double 
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
-        P.smem_blocks = smem_blocks(kThreads);
-        pdc::solve_scenes_kernel<kThreads><<<1, kThreads, smem_bytes(kThreads), st>>>(P, C);
+        const bool factor = cfg->sparse_max_bodies > 0;  // as in launch
+        P.smem_blocks = factor ? smem_blocks(kThreads) : 0;
+        pdc::solve_scenes_kernel<kThreads><<<1, kThreads, factor ? smem_bytes(kThreads) : 0, st>>>(P, C);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess)
