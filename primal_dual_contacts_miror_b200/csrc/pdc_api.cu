@@ -358,6 +358,32 @@ static cudaError_t allow_smem() {
     return e;
 }
 
+// The batched kernel on `grid` blocks, with the shared memory that a factor needs only
+// where there may be one: a handle that never factors leaves the L1 cache all of the
+// SM's, where the PCG of a scene of a few hundred bodies finds its contacts again every
+// iteration (pile of 200 boxes, 800 contacts, with these 70 KB per block and without:
+// 21.4 and 18.1 ms, mixed precision 20.3 and 13.6 ms).  For the same reason a launch with
+// no more blocks than SMs asks for one block's share of the SM, where the driver would
+// set aside what two blocks take (pile of 1,000 on PCG 120.1 -> 107.7 ms, 343 cubes
+// 59.7 -> 53.6 ms, pile of 500 in mixed precision 52.4 -> 48.2 ms; factors in global
+// memory gain too: crate of 144 5.83 -> 5.45 ms).
+static cudaError_t launch_solve(pdc::BatchPtrs P, const pdc::EngineCfg& C, int threads, int grid, int num_sms,
+                                bool factor, cudaStream_t st) {
+    P.smem_blocks = factor ? smem_blocks(threads) : 0;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[0].val.sharedMemCarveout = 36;  // % of 228 KB: 80 KB with the static part
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(threads);
+    lc.dynamicSmemBytes = factor ? smem_bytes(threads) : 0;
+    lc.stream = st;
+    lc.attrs = attr;
+    lc.numAttrs = factor && grid <= num_sms ? 1 : 0;
+    return threads == 128 ? cudaLaunchKernelEx(&lc, pdc::solve_scenes_kernel<128>, P, C)
+                          : cudaLaunchKernelEx(&lc, pdc::solve_scenes_kernel<256>, P, C);
+}
+
 extern "C" int pdc_create(const pdc_config* cfg, pdc_solver** out) {
     if (!out) return fail(nullptr, PDC_EINVAL, "null output handle");
     *out = nullptr;
@@ -493,15 +519,7 @@ static int launch(pdc_solver* s, const pdc::BatchPtrs& P0, cudaStream_t st, cons
     pdc::EngineCfg C = engine_cfg(s->cfg);
     pdc::plan_scenes_kernel<<<1, 1024, 0, st>>>(P, C);
     CK(cudaGetLastError(), "launch plan_scenes_kernel");
-    // A handle that never factors asks for no shared memory and leaves the L1 cache all
-    // of the SM's, where the PCG of a scene of a few hundred bodies finds its contacts
-    // again every iteration (pile of 200 boxes, 800 contacts, with these 70 KB per block
-    // and without: 21.4 and 18.1 ms, mixed precision 20.3 and 13.6 ms).
-    P.smem_blocks = P.dense ? smem_blocks(s->threads) : 0;
-    const size_t smem = P.dense ? smem_bytes(s->threads) : 0;
-    if (s->threads == 128) pdc::solve_scenes_kernel<128><<<grid, 128, smem, st>>>(P, C);
-    else pdc::solve_scenes_kernel<256><<<grid, 256, smem, st>>>(P, C);
-    CK(cudaGetLastError(), "launch solve_scenes_kernel");
+    CK(launch_solve(P, C, s->threads, grid, s->num_sms, P.dense != nullptr, st), "launch solve_scenes_kernel");
     if (P.grid_large) {
         if (!s->cluster_size) C.cluster_max_contacts = -1;
         for (int sc : *large) {
@@ -952,10 +970,7 @@ extern "C" int pdc_solve_noalloc(const pdc_config* cfg, double dt, const double 
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
-        const bool factor = cfg->sparse_max_bodies > 0;  // as in launch
-        P.smem_blocks = factor ? smem_blocks(kThreads) : 0;
-        pdc::solve_scenes_kernel<kThreads><<<1, kThreads, factor ? smem_bytes(kThreads) : 0, st>>>(P, C);
-        e = cudaGetLastError();
+        e = launch_solve(P, C, kThreads, 1, 1, cfg->sparse_max_bodies > 0, st);
     }
     if (e != cudaSuccess)
         return fail(nullptr, PDC_ECUDA, std::string("pdc_solve_noalloc: launch: ") + cudaGetErrorString(e));
